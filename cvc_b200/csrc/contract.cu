@@ -8,13 +8,24 @@
 //   sum_{g,ir,ia,ib} k(g,ir) us(ia,ib) [ chi_d(x)^+ g5 (g_mu - 1) U_mu(x) phi_c(x+mu)
 //                                       + chi_d(x+mu)^+ g5 (g_mu + 1) U_mu(x)^+ phi_c(x) ]
 // with c = (ir,ia), d = (gperm_g(ir), ib), k = +-1 or +-i and us an entry of
-// the (phased) source link.  The brackets are linear in chi, so the
-// coefficient sum can be moved onto the chi side once per site:
-//   Z_c(x) = sum_{g,ib} conj(k us) chi_{d(g,ir,ib)}(x)
-// after which Pi_mu_nu needs, per column c, one forward and one backward
-// hop of phi_c and two 12-component inner products with Z_c.  Kernel
-// k_cvc_z_sites (or k_cvc_z) builds the 24 Z columns of one nu (both parts);
-// k_cvc_pi does the hops and dots, accumulating in FP64 registers.
+// the (phased) source link.  Per part and nu the coefficients are K (x) us
+// with K = X_nu -+ g5, X_nu = g_nu g5, which has rank two like the vertex
+// (g_nu -+ 1) itself: its rows r and r' = partner of r are proportional.  One
+// of the two columns of a bracket belongs to the four shifted source points
+// (it depends on nu), the other to the source point itself (it does not).
+// k_pi therefore keeps the former local to the site a thread works on and
+// lets it meet the latter at the eight neighbours (the complex conjugate of
+// the bracket exchanges the roles for the second part):
+//   Z_{a,o}  = sum_i conj(Us_nu[o][i]) (f_{a,i}(x) - lam f_{a',i}(x)),  a = 0, 1
+//   u_{c,+-} = [half spinor of] (1 -+ g_mu) W g_c(x +- mu)
+//   T_{mu nu,+-}(x) = sum_{a,o} <Z_{a,o}, g5 (u_{(a,o),+-} + lam u_{(a',o),+-})>
+// with f the 12 columns of the point shifted by nu, g those of the source
+// point, and lam = conj(X_nu[a][a']) = +-1 or +-i, and
+//   Pi_mu_nu(x) = T_{mu nu,+}(x) - T_{mu nu,-}(x + mu),
+// T summed over the two parts (conjugated for the second).  (For the other
+// kernels of the path, which want the columns of all nu in the coefficient
+// form, k_cvc_z_sites or k_cvc_z builds the 24 columns
+// Z_c(x) = sum_{g,ib} conj(k us) chi_{d(g,ir,ib)}(x) of one nu.)
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -89,126 +100,261 @@ __global__ void __launch_bounds__(kZThreads) k_cvc_z_sites(double2 *__restrict__
   }
 }
 
-__device__ __forceinline__ Cx<double> dot_g5(const Spinor<double> &a, const Spinor<double> &b) {
-  // <a, g5 b> = sum over spins 0,1 of conj(a) b - sum over spins 2,3
-  Cx<double> p = cx(0.0, 0.0), m = cx(0.0, 0.0);
+// ---- the contraction kernel ------------------------------------------------
+// A block takes 8 consecutive lexicographic sites (V is a multiple of 16).
+// Per part it stages in shared memory the Z columns of all four nu (2 x 3
+// columns each, formed from the 48 shifted columns, every element read once
+// and coalesced although the fields are site-major) and the projected and
+// transported half spinors u of the 12 columns of the source point for the 8
+// neighbours; then each thread (colour of the sink, pair of nu with the same
+// spin partners, site, a, sign of the hop) forms its dots.  u is formed once
+// for all four nu, and the local columns need neither a copy in another
+// layout nor Z columns in memory.
+// Bounds at 24^3 x 48: 15.9 GB of compulsory traffic (2.4 ms at 6.55 TB/s) and
+// 42.6 k FP64 instructions per site (1.5 ms at 64 per SM and clock).  Measured
+// 7.5 ms (the whole contraction 9.2 ms; 44.6 ms with the columns copied to
+// component-major order, Z columns in memory and one thread per site; 0.27
+// against 2.41 ms at 8^3 x 16): load latency between the barriers at 12 warps
+// per SM bounds it (FP64 pipe 22 % busy).  Tried, no faster: all of a part's
+// local loads in flight at once and the links kept in registers (9.4 and
+// 9.7 ms), and bringing the next block's local columns to L2 (10.1 ms, DRAM
+// reads 1.5 times as many).
+constexpr int kPiSites = 8;
+constexpr int kPiThreads = 192;
+constexpr int kPiZ = 4 * 2 * 3 * 12 * kPiSites;  // double2: [nu][a][o][comp][site]
+constexpr int kPiU = 3 * 4 * 8 * 6 * kPiSites;   // double2: [ia][ir][dir][spin][colour][site]
+constexpr size_t kPiSmem = (kPiZ + kPiU) * sizeof(double2);
+
+struct PiArgs {
+  const double2 *loc[2][48];  // part 0: dn, part 1: up columns of the shifted points, site-major
+  const double2 *fix;         // [part][12 columns][12][V], lexicographic: columns of the source point
+  const double2 *U;
+  double2 *F, *B;   // T_+ and T_-, [V][mu][nu]
+  double2 us[4][9]; // conj of the phased source links
+  double lam[4][2]; // lam = lam (nu = 0, 2) or i lam (nu = 1, 3), per a
+  Geom g;
+};
+
+// slot of component comp of site s inside one Z column: the sites of a
+// component are permuted by it, so that both the writers (consecutive
+// components) and the readers (consecutive sites) spread over the banks
+__device__ __forceinline__ int z_slot(int comp, int s) { return comp * kPiSites + (s ^ (comp & 7)); }
+
+// u of one column and direction for the thread's site
+template <int MU, int S>
+__device__ __forceinline__ void pi_transport(const PiArgs &A, const SiteCoord &cd, int par,
+                                             const double2 *col, double2 *u) {
+  const Geom &g = A.g;
+  const int j = nb_lex(g, cd, MU, S < 0 ? +1 : -1);
+  Spinor<double> f;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    cfmac(p, a.c[0][c], b.c[0][c]);
-    cfmac(p, a.c[1][c], b.c[1][c]);
-    cfmac(m, a.c[2][c], b.c[2][c]);
-    cfmac(m, a.c[3][c], b.c[3][c]);
+  for (int k = 0; k < 12; ++k) {
+    const double2 v = __ldg(col + (size_t)k * g.V + j);
+    f.c[k / 3][k % 3] = cx(v.x, v.y);
   }
-  return p - m;
+  const int at = S < 0 ? par * g.Vh + (cd.lex >> 1) : (1 - par) * g.Vh + (j >> 1);
+  const Link<double> W = load_link64(A.U, g.V, MU, at);
+  const HalfSpinor<double> h = project(MU, S, f);
+  const HalfSpinor<double> r = S < 0 ? link_mul(W, h) : link_dag_mul(W, h);
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      u[(3 * b + c) * kPiSites] = make_double2(r.c[b][c].re, r.c[b][c].im);
 }
 
-__device__ __forceinline__ Spinor<double> recon_full(int mu, int s, const HalfSpinor<double> &u) {
-  Spinor<double> r;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) r.c[a][c] = cx(0.0, 0.0);
-  accum_recon(mu, s, r, u);
-  return r;
+// acc += conj(z) v
+__device__ __forceinline__ void dot_acc(Cx<double> &acc, Cx<double> z, Cx<double> v) {
+  cfmac(acc, z, v);
+}
+// z + s w and z + s i w
+__device__ __forceinline__ Cx<double> add_s(Cx<double> z, double s, Cx<double> w) {
+  return cx(fma(s, w.re, z.re), fma(s, w.im, z.im));
+}
+__device__ __forceinline__ Cx<double> add_si(Cx<double> z, double s, Cx<double> w) {
+  return cx(fma(-s, w.im, z.re), fma(s, w.re, z.im));
 }
 
-// Pi_mu_nu for one nu: P0 = up columns of part 0 (unshifted source),
-// P1 = up columns of part 1 (source shifted by nu), Z = 24 columns from
-// k_cvc_z.  conn is CVC layout (lexicographic, 32 doubles per site).
-// MINB: minimum resident blocks of 128 threads per SM, which caps the
-// registers (2: about 254, 8 warps per SM; 4: 128, 16 warps, a few spills);
-// the variant is chosen once per process by timing (cvc_pi_variant).
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) k_cvc_pi(double *__restrict__ conn,
-                                                const double2 *__restrict__ P0,
-                                                const double2 *__restrict__ P1,
-                                                const double2 *__restrict__ Z,
-                                                const double2 *__restrict__ U, Geom g, int nu) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.V) return;
-  const int p = s >= g.Vh;
-  const SiteCoord cd = site_coord(g, p, s - p * g.Vh);
-  const size_t V = g.V, fs = (size_t)12 * V;
-  const int qoff = (1 - p) * g.Vh;
-
-  Cx<double> pi[4];
-#pragma unroll
-  for (int mu = 0; mu < 4; ++mu) pi[mu] = cx(0.0, 0.0);
-
-#pragma unroll
-  for (int mu = 0; mu < 4; ++mu) {
-    const int j = qoff + (nb_lex(g, cd, mu, +1) >> 1);
-    const Link<double> W = load_link64(U, V, mu, s);
-    for (int part = 0; part < 2; ++part) {
-      const double2 *P = part == 0 ? P0 : P1;
-      for (int c = 0; c < 12; ++c) {
-        const double2 *Pc = P + c * fs;
-        const double2 *Zc = Z + (part * 12 + c) * fs;
-        // forward: g5 (g_mu - 1) U_mu(x) P_c(x+mu) = -g5 (1 - g_mu) U P
-        {
-          const HalfSpinor<double> h = project(mu, -1, load_spinor(Pc, V, j));
-          const Spinor<double> r = recon_full(mu, -1, link_mul(W, h));
-          const Cx<double> w = dot_g5(load_spinor(Zc, V, s), r);
-          pi[mu] = pi[mu] - w;
-        }
-        // backward: g5 (g_mu + 1) U_mu(x)^+ P_c(x), dotted with Z_c(x+mu)
-        {
-          const HalfSpinor<double> h = project(mu, +1, load_spinor(Pc, V, s));
-          const Spinor<double> r = recon_full(mu, +1, link_dag_mul(W, h));
-          const Cx<double> w = dot_g5(load_spinor(Zc, V, j), r);
-          pi[mu] = pi[mu] + w;
-        }
-      }
-    }
+__global__ void __launch_bounds__(kPiThreads, 2) k_pi(const __grid_constant__ PiArgs A) {
+  extern __shared__ double2 sm[];
+  double2 *sz = sm, *su = sm + kPiZ;
+  const Geom &g = A.g;
+  const int base = blockIdx.x * kPiSites;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int site = lane & 7;
+  SiteCoord cd;
+  {
+    cd.lex = base + site;
+    const unsigned r0 = fdiv((unsigned)cd.lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
+    cd.z = cd.lex - (int)r0 * g.LZ;
+    cd.y = (int)(r0 - r1 * g.LY);
+    cd.x = (int)(r1 - r2 * g.LX);
+    cd.t = (int)r2;
   }
-  double *o = conn + (size_t)cd.lex * 32;
+  const int par = (cd.t + cd.x + cd.y + cd.z) & 1;
+  // the dots' role of the thread
+  const int si = warp % 3, cls = warp / 3;           // colour of the sink; nu in {0,3} or {2,1}
+  const int a = (lane >> 3) & 1, sg = lane >> 4;     // source spin; forward or backward hop
+  const int ap = cls == 0 ? a + 2 : 3 - a;           // its partner
+  const int nur = cls == 0 ? 0 : 2, nui = cls == 0 ? 3 : 1;
+  const double lr = A.lam[nur][a], li = A.lam[nui][a];
+  const double s = sg ? 1.0 : -1.0;
+  Cx<double> acc[2][4];
 #pragma unroll
-  for (int mu = 0; mu < 4; ++mu) {
-    o[2 * (4 * mu + nu)] = -0.25 * pi[mu].re;  // normalisation, :861
-    o[2 * (4 * mu + nu) + 1] = -0.25 * pi[mu].im;
-  }
-}
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int mu = 0; mu < 4; ++mu) acc[n][mu] = cx(0.0, 0.0);
 
-// The same Pi_mu_nu with one thread per (site, mu), mu = blockIdx.y: four
-// times the threads, each with one link and a quarter of the loop (no
-// unrolled mu loop holding its state), so that more warps fit under the
-// same register cap.  Each thread accumulates pi_mu over (part, c) in the
-// order of k_cvc_pi and writes only its own mu entry: the same bits.
-template <int MINB>
-__global__ void __launch_bounds__(128, MINB) k_cvc_pi_mu(double *__restrict__ conn,
-                                                   const double2 *__restrict__ P0,
-                                                   const double2 *__restrict__ P1,
-                                                   const double2 *__restrict__ Z,
-                                                   const double2 *__restrict__ U, Geom g, int nu) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.V) return;
-  const int mu = blockIdx.y;
-  const int p = s >= g.Vh;
-  const SiteCoord cd = site_coord(g, p, s - p * g.Vh);
-  const size_t V = g.V, fs = (size_t)12 * V;
-  const int j = (1 - p) * g.Vh + (nb_lex(g, cd, mu, +1) >> 1);
-  const Link<double> W = load_link64(U, V, mu, s);
-  Cx<double> pi = cx(0.0, 0.0);
+#pragma unroll 1
   for (int part = 0; part < 2; ++part) {
-    const double2 *P = part == 0 ? P0 : P1;
-    for (int c = 0; c < 12; ++c) {
-      const double2 *Pc = P + c * fs;
-      const double2 *Zc = Z + (part * 12 + c) * fs;
-      {  // forward: g5 (g_mu - 1) U_mu(x) P_c(x+mu), dotted with Z_c(x)
-        const HalfSpinor<double> h = project(mu, -1, load_spinor(Pc, V, j));
-        const Spinor<double> r = recon_full(mu, -1, link_mul(W, h));
-        pi = pi - dot_g5(load_spinor(Zc, V, s), r);
+    // Z: 8 (nu, a) x 96 elements (site, component), six columns in, three out
+#pragma unroll 1
+    for (int q = warp; q < 24; q += kPiThreads / 32) {
+      const int na = q / 3, nu = na >> 1, za = na & 1;
+      const int zp = nu == 0 || nu == 3 ? za + 2 : 3 - za;
+      const int e = (q % 3) * 32 + lane, es = e / 12, ec = e - 12 * es;
+      const size_t off = (size_t)base * 12 + e;
+      const double l = A.lam[nu][za];
+      Cx<double> y[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const double2 v = __ldg(A.loc[part][12 * nu + 3 * za + i] + off);
+        const double2 w = __ldg(A.loc[part][12 * nu + 3 * zp + i] + off);
+        y[i] = nu & 1 ? add_si(cx(v.x, v.y), -l, cx(w.x, w.y)) : add_s(cx(v.x, v.y), -l, cx(w.x, w.y));
       }
-      {  // backward: g5 (g_mu + 1) U_mu(x)^+ P_c(x), dotted with Z_c(x+mu)
-        const HalfSpinor<double> h = project(mu, +1, load_spinor(Pc, V, s));
-        const Spinor<double> r = recon_full(mu, +1, link_dag_mul(W, h));
-        pi = pi + dot_g5(load_spinor(Zc, V, j), r);
+#pragma unroll
+      for (int o = 0; o < 3; ++o) {
+        Cx<double> z = cx(0.0, 0.0);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) cfma(z, cx(A.us[nu][3 * o + i].x, A.us[nu][3 * o + i].y), y[i]);
+        sz[(na * 3 + o) * 12 * kPiSites + z_slot(ec, es)] = make_double2(z.re, z.im);
       }
     }
+    // u: 8 directions x 3 colours, lanes = 8 sites x 4 source spins
+#pragma unroll 1
+    for (int q = warp; q < 24; q += kPiThreads / 32) {
+      const int dir = q / 3, ia = q % 3, ir = lane >> 3;
+      const double2 *col = A.fix + (size_t)(part * 12 + 3 * ir + ia) * 12 * g.V;
+      double2 *u = su + ((ia * 4 + ir) * 8 + dir) * 6 * kPiSites + site;
+      switch (dir) {
+        case 0: pi_transport<0, -1>(A, cd, par, col, u); break;
+        case 1: pi_transport<1, -1>(A, cd, par, col, u); break;
+        case 2: pi_transport<2, -1>(A, cd, par, col, u); break;
+        case 3: pi_transport<3, -1>(A, cd, par, col, u); break;
+        case 4: pi_transport<0, +1>(A, cd, par, col, u); break;
+        case 5: pi_transport<1, +1>(A, cd, par, col, u); break;
+        case 6: pi_transport<2, +1>(A, cd, par, col, u); break;
+        default: pi_transport<3, +1>(A, cd, par, col, u); break;
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int o = 0; o < 3; ++o) {
+      Cx<double> zr[4], zi[4];
+#pragma unroll
+      for (int sp = 0; sp < 4; ++sp) {
+        const int sl = z_slot(3 * sp + si, site);
+        const double2 v = sz[((nur * 2 + a) * 3 + o) * 12 * kPiSites + sl];
+        const double2 w = sz[((nui * 2 + a) * 3 + o) * 12 * kPiSites + sl];
+        zr[sp] = cx(v.x, v.y);
+        zi[sp] = cx(w.x, w.y);
+      }
+#pragma unroll
+      for (int mu = 0; mu < 4; ++mu) {
+        const int d = sg * 4 + mu;
+        const double2 *u1 = su + (((o * 4 + a) * 8 + d) * 6 + si) * kPiSites + site;
+        const double2 *u2 = su + (((o * 4 + ap) * 8 + d) * 6 + si) * kPiSites + site;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const double2 p = u1[3 * b * kPiSites], q = u2[3 * b * kPiSites];
+          const Cx<double> vr = add_s(cx(p.x, p.y), lr, cx(q.x, q.y));
+          const Cx<double> vi = add_si(cx(p.x, p.y), li, cx(q.x, q.y));
+          // the conjugate-transposed reconstruction of spins 2, 3 with g5
+          const int hi = mu == 0 || mu == 3 ? 2 + b : 3 - b;
+          const double sb = (mu >= 2 && b == 1) ? -s : s;
+          const bool im = mu & 1;
+          dot_acc(acc[0][mu], im ? add_si(zr[b], sb, zr[hi]) : add_s(zr[b], sb, zr[hi]), vr);
+          dot_acc(acc[1][mu], im ? add_si(zi[b], sb, zi[hi]) : add_s(zi[b], sb, zi[hi]), vi);
+        }
+      }
+    }
+    __syncthreads();
+    // the second part enters conjugated: conj(conj(T_0) + T_1)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int mu = 0; mu < 4; ++mu) acc[n][mu].im = -acc[n][mu].im;
   }
-  double *o = conn + (size_t)cd.lex * 32;
-  o[2 * (4 * mu + nu)] = -0.25 * pi.re;  // normalisation, :861
-  o[2 * (4 * mu + nu) + 1] = -0.25 * pi.im;
+  // sum over a (lanes) and the sink's colour (warps), in a fixed order
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int mu = 0; mu < 4; ++mu) {
+      Cx<double> t = acc[n][mu];
+      t.re += __shfl_xor_sync(0xffffffffu, t.re, 8);
+      t.im += __shfl_xor_sync(0xffffffffu, t.im, 8);
+      if (a == 0)
+        sm[((si * 8 + sg * 4 + mu) * 4 + (n ? nui : nur)) * kPiSites + site] = make_double2(t.re, t.im);
+    }
+  __syncthreads();
+  for (int k = threadIdx.x; k < 256; k += kPiThreads) {
+    const int ks = (k >> 4) & 7, slot = (((k >> 7) * 4 + ((k >> 2) & 3)) * 4 + (k & 3)) * kPiSites + ks;
+    const double2 x = sm[slot], y = sm[slot + 32 * kPiSites], z = sm[slot + 64 * kPiSites];
+    double2 *o = (k >> 7) ? A.B : A.F;
+    o[(size_t)(base + ks) * 16 + (k & 15)] = make_double2(x.x + y.x + z.x, x.y + y.y + z.y);
+  }
+}
+
+// conn_mu_nu(x) = -1/4 (T_+(x) - T_-(x + mu))   (normalisation, :861)
+__global__ void k_pi_combine(double2 *__restrict__ conn, const double2 *__restrict__ F,
+                             const double2 *__restrict__ B, Geom g) {
+  const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (k >= (size_t)g.V * 16) return;
+  SiteCoord cd;
+  cd.lex = (int)(k >> 4);
+  const unsigned r0 = fdiv((unsigned)cd.lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
+  cd.z = cd.lex - (int)r0 * g.LZ;
+  cd.y = (int)(r0 - r1 * g.LY);
+  cd.x = (int)(r1 - r2 * g.LX);
+  cd.t = (int)r2;
+  const int m = (int)(k & 15);
+  const double2 f = F[k], b = B[(size_t)nb_lex(g, cd, m >> 2, +1) * 16 + m];
+  conn[k] = make_double2(-0.25 * (f.x - b.x), -0.25 * (f.y - b.y));
+}
+
+// columns of the source point from CVC layout to component-major:
+// dst[column][component][V], lexicographic
+struct FixCols {
+  const double2 *src[24];
+};
+constexpr int kFixTile = 64;
+__global__ void __launch_bounds__(128) k_fix_columns(double2 *__restrict__ dst,
+                                                    const __grid_constant__ FixCols c, int V) {
+  __shared__ double2 t[kFixTile * 13];
+  const int base = blockIdx.x * kFixTile, n = min(kFixTile, V - base);
+  const double2 *src = c.src[blockIdx.y] + (size_t)base * 12;
+  for (int q = threadIdx.x; q < n * 12; q += blockDim.x) {
+    const int s = q / 12;
+    t[q + s] = __ldg(src + q);
+  }
+  __syncthreads();
+  double2 *d = dst + (size_t)blockIdx.y * 12 * V + base;
+  for (int q = threadIdx.x; q < kFixTile * 12; q += blockDim.x) {
+    const int k = q / kFixTile, s = q % kFixTile;
+    if (s < n) d[(size_t)k * V + s] = t[s * 13 + k];
+  }
+}
+
+// the 96 spinors of the contact term (:697-704, :837-844)
+struct ContactCols {
+  const double *src[60];  // up columns
+  int iup[4], site;
+};
+__global__ void k_contact_gather(double *__restrict__ out, const __grid_constant__ ContactCols c) {
+  const int q = blockIdx.x, part = q / 48, nu = (q / 12) % 4, col = q % 12;
+  const double *f = part == 0 ? c.src[48 + col] : c.src[nu * 12 + col];
+  if (threadIdx.x < 24)
+    out[q * 24 + threadIdx.x] = f[24 * (size_t)(part == 0 ? c.iup[nu] : c.site) + threadIdx.x];
 }
 
 // Ward identity divergence on the CVC-layout conn (cvc_exact2_xspace.c:938-953)
@@ -324,6 +470,19 @@ struct LinkSumF {
   }
 };
 
+// phased source links Usource[nu] (cvc_exact2_xspace.c:293-304)
+static void source_links(const cvcb_lattice *L, int src, double Us[4][18]) {
+  const double *G = L->gauge_host.data();
+  for (int nu = 0; nu < 4; ++nu)
+    for (int k = 0; k < 9; ++k) {
+      const double re = G[18 * (4 * (size_t)src + nu) + 2 * k],
+                   im = G[18 * (4 * (size_t)src + nu) + 2 * k + 1];
+      const double pr = L->phase[2 * nu], pi = L->phase[2 * nu + 1];
+      Us[nu][2 * k] = re * pr - im * pi;
+      Us[nu][2 * k + 1] = re * pi + im * pr;
+    }
+}
+
 // Coefficient plans of the Z columns for the four nu (see the file comment),
 // and the phased source links Usource[nu] (cvc_exact2_xspace.c:293-304).
 int make_zplans(cvcb_lattice *L, int src, ZPlan plans[4], double Us[4][18], ZMeta *meta) {
@@ -343,17 +502,7 @@ int make_zplans(cvcb_lattice *L, int src, ZPlan plans[4], double Us[4][18], ZMet
     }
     isimag[nu] = perm[6 + nu][0] % 2;
   }
-  // phased source links Usource[nu] (:293-304)
-  const double *G = L->gauge_host.data();
-  for (int nu = 0; nu < 4; ++nu)
-    for (int k = 0; k < 9; ++k) {
-      const double re = G[18 * (4 * (size_t)src + nu) + 2 * k],
-                   im = G[18 * (4 * (size_t)src + nu) + 2 * k + 1];
-      const double pr = L->phase[2 * nu], pi = L->phase[2 * nu + 1];
-      Us[nu][2 * k] = re * pr - im * pi;
-      Us[nu][2 * k + 1] = re * pi + im * pr;
-    }
-
+  source_links(L, src, Us);
   for (int nu = 0; nu < 4; ++nu) {
     ZPlan &plan = plans[nu];
     for (int part = 0; part < 2; ++part)
@@ -440,16 +589,6 @@ static int need_gauge(cvcb_lattice *L) {
   return CVCB_OK;
 }
 
-// Copy the Pi buffer (CVC layout on the device) to the caller.
-static int conn_out(cvcb_lattice *L, double *dst, const double *src, size_t ndouble) {
-  CVCB_CUDA(cudaMemcpyAsync(dst, src, ndouble * sizeof(double), cudaMemcpyDefault, L->stream));
-  return CVCB_OK;
-}
-
-// Variant of the Pi kernel (0-2: k_cvc_pi at 2, 3, 4 blocks per SM; 3-5:
-// k_cvc_pi_mu likewise), timed on first use; CVCB_CVC_PI=v pins it.
-static int g_cvc_pi_variant = -1;
-
 int cvc_contract(cvcb_lattice *L, const double *const *fields, int src, double *conn,
                  double *contact) {
   CVCB_TRY(need_gauge(L));
@@ -458,91 +597,108 @@ int cvc_contract(cvcb_lattice *L, const double *const *fields, int src, double *
     set_error("source site %d outside [0, %d)", src, g.V);
     return CVCB_ERR_ARG;
   }
-  for (int f = 0; f < 120; ++f)
+  int nhost = 0;
+  bool on_host[120];
+  for (int f = 0; f < 120; ++f) {
     if (!fields[f]) {
       set_error("field %d is NULL", f);
       return CVCB_ERR_NULL;
     }
+    on_host[f] = !is_device_ptr(fields[f]);
+    nhost += on_host[f];
+  }
   const size_t fs = (size_t)12 * g.V;  // double2 per field
-  void *props, *zb, *cb;
-  CVCB_TRY(ensure_buffer(L, SLOT_PROPS, 120 * fs * sizeof(double2), &props));
-  CVCB_TRY(ensure_buffer(L, SLOT_F2, 24 * fs * sizeof(double2), &zb));
-  CVCB_TRY(ensure_buffer(L, SLOT_CONN, (size_t)g.V * 32 * sizeof(double), &cb));
-  double2 *P = static_cast<double2 *>(props);
-  for (int f = 0; f < 120; ++f) CVCB_TRY(spinor_in(L, P + f * fs, fields[f], g.V));
+  void *fixb, *cb, *hb = nullptr;
+  if (nhost) CVCB_TRY(ensure_buffer(L, SLOT_PROPS, nhost * fs * sizeof(double2), &hb));
+  CVCB_TRY(ensure_buffer(L, SLOT_F2, 24 * fs * sizeof(double2), &fixb));
+  // T_+, T_-, and the contact term's spinors
+  const size_t piv = (size_t)g.V * 16;
+  CVCB_TRY(ensure_buffer(L, SLOT_CONN, 2 * piv * sizeof(double2) + 96 * 24 * sizeof(double), &cb));
+  const double *dev[120];
+  for (int f = 0, h = 0; f < 120; ++f) {
+    dev[f] = fields[f];
+    if (on_host[f]) {
+      double2 *d = static_cast<double2 *>(hb) + fs * h++;
+      CVCB_CUDA(cudaMemcpyAsync(d, fields[f], fs * sizeof(double2), cudaMemcpyHostToDevice,
+                                L->stream));
+      dev[f] = reinterpret_cast<const double *>(d);
+    }
+  }
 
-  ZPlan plans[4];
-  double Us[4][18];
+  // phased source links Usource[nu] (:293-304) and the spin structure of the vertex
   int perm[16][24], sign[16][24];
   gamma_tables(perm, sign);
-  make_zplans(L, src, plans, Us, nullptr);
-  const int blocks = (g.V + 127) / 128;
-  auto pi = [&](int v, int nu) {
-    double *c = static_cast<double *>(cb);
-    const double2 *P1 = P + (size_t)nu * 12 * fs, *Z = static_cast<const double2 *>(zb);
-    const dim3 gmu(blocks, 4);  // k_cvc_pi_mu: one thread per (site, mu)
-    switch (v) {
-      case 1: k_cvc_pi<3><<<blocks, 128, 0, L->stream>>>(c, P + 48 * fs, P1, Z, L->U64, g, nu); break;
-      case 2: k_cvc_pi<4><<<blocks, 128, 0, L->stream>>>(c, P + 48 * fs, P1, Z, L->U64, g, nu); break;
-      case 3: k_cvc_pi_mu<2><<<gmu, 128, 0, L->stream>>>(c, P + 48 * fs, P1, Z, L->U64, g, nu); break;
-      case 4: k_cvc_pi_mu<3><<<gmu, 128, 0, L->stream>>>(c, P + 48 * fs, P1, Z, L->U64, g, nu); break;
-      case 5: k_cvc_pi_mu<4><<<gmu, 128, 0, L->stream>>>(c, P + 48 * fs, P1, Z, L->U64, g, nu); break;
-      default: k_cvc_pi<2><<<blocks, 128, 0, L->stream>>>(c, P + 48 * fs, P1, Z, L->U64, g, nu); break;
-    }
-  };
+  double Us[4][18];
+  source_links(L, src, Us);
+  PiArgs A;
+  FixCols fc;
   for (int nu = 0; nu < 4; ++nu) {
-    CVCB_TRY(launch_cvc_z(L, static_cast<double2 *>(zb), P + 60 * fs, plans[nu]));
-    if (g_cvc_pi_variant < 0)
-      if (const char *env = getenv("CVCB_CVC_PI")) {
-        const int v = atoi(env);
-        if (v >= 0 && v < 6) g_cvc_pi_variant = v;
+    for (int k = 0; k < 9; ++k) A.us[nu][k] = make_double2(Us[nu][2 * k], -Us[nu][2 * k + 1]);
+    for (int a = 0; a < 2; ++a) {
+      const int ap = nu == 0 || nu == 3 ? a + 2 : 3 - a, *pm = perm[6 + nu] + 6 * a;
+      const bool imag = pm[0] % 2;
+      if (pm[0] / 6 != ap || imag != (bool)(nu & 1)) {  // the kernel's table of partners
+        set_error("unexpected gamma table");
+        return CVCB_ERR_STATE;
       }
-    if (g_cvc_pi_variant < 0) {  // first use in this process: time the variants (same results)
-      cudaEvent_t e0, e1;
-      CVCB_CUDA(cudaEventCreate(&e0));
-      CVCB_CUDA(cudaEventCreate(&e1));
-      float best = 1e30f;
-      for (int v = 0; v < 6; ++v) {
-        CVCB_CUDA(cudaEventRecord(e0, L->stream));
-        pi(v, nu);
-        CVCB_CUDA(cudaEventRecord(e1, L->stream));
-        CVCB_CUDA(cudaEventSynchronize(e1));
-        float ms;
-        CVCB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best) best = ms, g_cvc_pi_variant = v;
-      }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
+      // lam = conj(X_nu[a][a']), X = sign (real) or -i sign (imaginary)
+      A.lam[nu][a] = sign[6 + nu][6 * a];
     }
-    pi(g_cvc_pi_variant, nu);
+  }
+  for (int c = 0; c < 48; ++c) {
+    A.loc[0][c] = reinterpret_cast<const double2 *>(dev[60 + c]);
+    A.loc[1][c] = reinterpret_cast<const double2 *>(dev[c]);
+  }
+  for (int c = 0; c < 12; ++c) {
+    fc.src[c] = reinterpret_cast<const double2 *>(dev[48 + c]);
+    fc.src[12 + c] = reinterpret_cast<const double2 *>(dev[108 + c]);
+  }
+  A.fix = static_cast<const double2 *>(fixb);
+  A.U = L->U64;
+  A.F = static_cast<double2 *>(cb);
+  A.B = A.F + piv;
+  A.g = g;
+  k_fix_columns<<<dim3((g.V + kFixTile - 1) / kFixTile, 24), 128, 0, L->stream>>>(
+      static_cast<double2 *>(fixb), fc, g.V);
+  CVCB_LAUNCHED(L);
+  CVCB_CUDA(cudaFuncSetAttribute(k_pi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPiSmem));
+  k_pi<<<g.V / kPiSites, kPiThreads, kPiSmem, L->stream>>>(A);
+  CVCB_LAUNCHED(L);
+  // contact term (:697-704, :837-844) from a handful of spinors
+  double *ctb = reinterpret_cast<double *>(A.B + piv);
+  std::vector<double> sp;
+  if (contact) {
+    sp.resize(96 * 24);
+    ContactCols cc;
+    for (int c = 0; c < 60; ++c) cc.src[c] = dev[c];
+    const int z = src % g.LZ, y = (src / g.LZ) % g.LY, x = (src / g.s2) % g.LX, t = src / g.s3;
+    cc.iup[0] = ((t + 1) % g.T) * g.s3 + x * g.s2 + y * g.s1 + z;
+    cc.iup[1] = t * g.s3 + ((x + 1) % g.LX) * g.s2 + y * g.s1 + z;
+    cc.iup[2] = t * g.s3 + x * g.s2 + ((y + 1) % g.LY) * g.s1 + z;
+    cc.iup[3] = t * g.s3 + x * g.s2 + y * g.s1 + (z + 1) % g.LZ;
+    cc.site = src;
+    k_contact_gather<<<96, 32, 0, L->stream>>>(ctb, cc);
     CVCB_LAUNCHED(L);
   }
-  CVCB_TRY(conn_out(L, conn, static_cast<const double *>(cb), (size_t)g.V * 32));
-
+  // Pi in CVC layout straight into the caller's array where that is memory of
+  // this device on a 16-byte boundary, else through the (spent) column buffer
+  const bool direct = is_own_device_ptr(L, conn) && (reinterpret_cast<uintptr_t>(conn) & 15) == 0;
+  double2 *out = direct ? reinterpret_cast<double2 *>(conn) : static_cast<double2 *>(fixb);
+  k_pi_combine<<<(int)((piv + 255) / 256), 256, 0, L->stream>>>(out, A.F, A.B, g);
+  CVCB_LAUNCHED(L);
+  if (!direct)
+    CVCB_CUDA(cudaMemcpyAsync(conn, out, piv * sizeof(double2), cudaMemcpyDefault, L->stream));
+  if (contact)
+    CVCB_CUDA(cudaMemcpyAsync(sp.data(), ctb, sp.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                              L->stream));
+  CVCB_CUDA(cudaStreamSynchronize(L->stream));
   if (contact) {
-    // contact term (:697-704, :837-844) from a handful of spinors
-    std::vector<double> sp(24);
     double ct[8] = {0};
-    int iup[4];
-    {
-      const int z = src % g.LZ, y = (src / g.LZ) % g.LY, x = (src / g.s2) % g.LX, t = src / g.s3;
-      iup[0] = ((t + 1) % g.T) * g.s3 + x * g.s2 + y * g.s1 + z;
-      iup[1] = t * g.s3 + ((x + 1) % g.LX) * g.s2 + y * g.s1 + z;
-      iup[2] = t * g.s3 + x * g.s2 + ((y + 1) % g.LY) * g.s1 + z;
-      iup[3] = t * g.s3 + x * g.s2 + y * g.s1 + (z + 1) % g.LZ;
-    }
-    auto fetch = [&](const double *f, int site, double *out24) -> int {
-      CVCB_CUDA(cudaMemcpyAsync(out24, f + 24 * (size_t)site, 24 * sizeof(double),
-                                cudaMemcpyDefault, L->stream));
-      return CVCB_OK;
-    };
     for (int part = 0; part < 2; ++part)
       for (int nu = 0; nu < 4; ++nu)
         for (int ir = 0; ir < 4; ++ir)
           for (int ia = 0; ia < 3; ++ia) {
-            const double *phi = part == 0 ? fields[48 + 3 * ir + ia] : fields[nu * 12 + 3 * ir + ia];
-            CVCB_TRY(fetch(phi, part == 0 ? iup[nu] : src, sp.data()));
-            CVCB_CUDA(cudaStreamSynchronize(L->stream));
+            const double *phi = sp.data() + 24 * ((part * 4 + nu) * 12 + 3 * ir + ia);
             double s1[24], s2[24];
             for (int a = 0; a < 4; ++a)
               for (int i = 0; i < 3; ++i) {
@@ -552,7 +708,7 @@ int cvc_contract(cvcb_lattice *L, const double *const *fields, int src, double *
                   double ur, ui;
                   if (part == 0) { ur = Us[nu][2 * (3 * i + j)]; ui = Us[nu][2 * (3 * i + j) + 1]; }
                   else { ur = Us[nu][2 * (3 * j + i)]; ui = -Us[nu][2 * (3 * j + i) + 1]; }
-                  const double vr = sp[2 * (3 * a + j)], vi = sp[2 * (3 * a + j) + 1];
+                  const double vr = phi[2 * (3 * a + j)], vi = phi[2 * (3 * a + j) + 1];
                   re += ur * vr - ui * vi;
                   im += ur * vi + ui * vr;
                 }
@@ -571,7 +727,6 @@ int cvc_contract(cvcb_lattice *L, const double *const *fields, int src, double *
           }
     std::memcpy(contact, ct, sizeof ct);
   }
-  CVCB_CUDA(cudaStreamSynchronize(L->stream));
   return CVCB_OK;
 }
 

@@ -224,6 +224,7 @@ constexpr int kMaxRedBlocks = 1184;  // 8 x 148 SMs
 // lattice.cu
 int ensure_buffer(cvcb_lattice *L, int slot, size_t bytes, void **out);
 bool is_device_ptr(const void *p);
+bool is_own_device_ptr(const cvcb_lattice *L, const void *p);  // memory of the lattice's GPU
 // Copy a CVC-layout FP64 spinor (host or device) into device layout `dst`.
 int spinor_in(cvcb_lattice *L, double2 *dst, const double *src, int nsites_aos);
 // Copy device-layout `src` into a CVC-layout FP64 spinor (host or device).

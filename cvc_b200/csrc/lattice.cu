@@ -29,6 +29,15 @@ bool is_device_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+bool is_own_device_ptr(const cvcb_lattice *L, const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == L->device;
+}
+
 int ensure_buffer(cvcb_lattice *L, int slot, size_t bytes, void **out) {
   if ((int)L->bufs.size() <= slot) L->bufs.resize(slot + 1);
   Buffer &b = L->bufs[slot];

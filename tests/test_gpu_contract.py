@@ -93,6 +93,36 @@ def test_seq_source(env, t, mom, gid, pos):
     assert rel_err(src, ref) < 1e-14
 
 
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 4, 2, 6), (6, 2, 10, 2), (4, 6, 2, 18)],
+                         ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("where", ["host", "device", "mixed"])
+def test_contract_shapes(cb, oracle_mod, dims, where):
+    """Extents of two (both hops reach the same site) and z extents that cut a
+    block's run of 8 sites, with fields on the host, on the device and on
+    both, and Pi into device memory off a 16-byte boundary.  Sums of some
+    4608 terms of rounding 2^-53 each: 1e-12 of the largest entry."""
+    torch = pytest.importorskip("torch")
+    bc = (1.0, 0.3, 0.0, 0.5)
+    lat = cb.Lattice(*dims, kappa=KAPPA, mu=MU, bc_angle=bc)
+    V = lat.VOLUME
+    g = cb.gauge_random(*dims, 0.3, 5)
+    lat.upload_gauge(g)
+    orc = oracle_mod.Oracle(*dims, KAPPA, MU, bc)
+    orc.set_gauge(g)
+    fields = [seeded(50 + i, 24 * V) for i in range(120)]
+    src = V // 2 + 1
+    oconn, ocontact = orc.cvc_contract(fields, src)
+    given = [torch.from_numpy(f).cuda() if where == "device" or (where == "mixed" and i % 3)
+             else f for i, f in enumerate(fields)]
+    torch.cuda.synchronize()
+    out = None if where == "host" else torch.zeros(32 * V + 1, dtype=torch.float64, device="cuda")[1:]
+    conn, contact = lat.cvc_contract(given, src, conn=out)
+    conn = conn if where == "host" else conn.cpu().numpy()
+    assert rel_err(conn, oconn) < 1e-12
+    assert np.max(np.abs(contact - ocontact)) < 1e-12 * np.max(np.abs(ocontact))
+    lat.close()
+
+
 VARIANT_CHILD = r"""
 import sys
 import numpy as np
