@@ -55,6 +55,40 @@ def test_against_numpy(lat, src, with_contact):
     assert rel_err(got, numpy_pi_momentum(conn, src, contact)) < 1e-13
 
 
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (22, 2, 26, 4), (34, 2, 4, 6), (4, 6, 2, 34),
+                                  (2, 2, 72, 128), (64, 16, 2, 2)],
+                         ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("where", ["host", "device", "odd"])
+def test_shapes(cb, dims, where):
+    """Extents with factors up to 8, up to 16 and above (17: one direction a
+    pass), a plane too large for shared memory, and arrays on the host, on
+    the device and off a 16-byte boundary, in and out the same array.  Sums
+    of V terms in stages of rounding 2^-53: 1e-13 as above."""
+    torch = pytest.importorskip("torch")
+    lt = cb.Lattice(*dims, kappa=KAPPA, mu=MU)
+    n = lt.VOLUME
+    conn, contact, src = seeded(11, 32 * n), seeded(12, 8), n // 2 + 1
+    z = (conn[0::2] + 1j * conn[1::2]).reshape(*dims, 4, 4)
+    F = np.fft.fftn(z, axes=(0, 1, 2, 3))
+    q = np.meshgrid(*[2 * np.pi * np.arange(L) / L for L in dims], indexing="ij")
+    qy = sum(a * c for a, c in zip(q, np.unravel_index(src, dims)))
+    for mu in range(4):
+        for nu in range(4):
+            F[..., mu, nu] *= np.exp(1j * (qy - 0.5 * q[mu] + 0.5 * q[nu]))
+        F[..., mu, mu] -= contact[2 * mu] + 1j * contact[2 * mu + 1]
+    want = np.stack([F.real.ravel(), F.imag.ravel()], 1).ravel()
+    if where == "host":
+        got = lt.pi_momentum(conn, src, contact)
+    else:
+        d = torch.zeros(32 * n + 2, dtype=torch.float64, device="cuda")
+        d = d[1:32 * n + 1] if where == "odd" else d[:32 * n]
+        d.copy_(torch.from_numpy(conn))
+        torch.cuda.synchronize()
+        got = lt.pi_momentum(d, src, contact, out=d).cpu().numpy()
+    assert rel_err(got, want) < 1e-13
+    lt.close()
+
+
 def test_device_pointers(lat):
     torch = pytest.importorskip("torch")
     conn = seeded(3, 32 * V)
