@@ -47,20 +47,31 @@ int need_gauge(cvcb_lattice *L) {
   return CVCB_OK;
 }
 
-// out = op(in) with the full-lattice kernel; in/out in CVC layout.
+// out = op(in) with the full-lattice kernel on CVC-layout fields, in place on
+// device arrays; host arrays go through staging, and so does an input that
+// overlaps the output.
 int apply_full(cvcb_lattice *L, double *xi, const double *phi, double a, double b, double c,
                bool g5out) {
   CVCB_TRY(need_gauge(L));
   if (!xi || !phi) return CVCB_ERR_NULL;
   CVCB_CUDA(cudaSetDevice(L->device));
-  const size_t fb = (size_t)L->g.V * 12 * sizeof(double2);
-  void *f0, *f1;
-  CVCB_TRY(ensure_buffer(L, SLOT_F0, fb, &f0));
-  CVCB_TRY(ensure_buffer(L, SLOT_F1, fb, &f1));
-  CVCB_TRY(spinor_in(L, static_cast<double2 *>(f0), phi, L->g.V));
-  CVCB_TRY(launch_tm_full(L, static_cast<double2 *>(f1), static_cast<const double2 *>(f0), a, b,
-                          c, g5out, nullptr));
-  CVCB_TRY(spinor_out(L, xi, static_cast<const double2 *>(f1), L->g.V));
+  const size_t n = (size_t)L->g.V * 24, fb = n * sizeof(double);
+  const uintptr_t x = reinterpret_cast<uintptr_t>(xi), p = reinterpret_cast<uintptr_t>(phi);
+  const bool out_dev = is_device_ptr(xi);
+  const double *in = phi;
+  double *out = xi;
+  void *f;
+  if (!is_device_ptr(phi) || (out_dev && x < p + fb && p < x + fb)) {
+    CVCB_TRY(ensure_buffer(L, SLOT_F0, fb, &f));
+    CVCB_CUDA(cudaMemcpyAsync(f, phi, fb, cudaMemcpyDefault, L->stream));
+    in = static_cast<const double *>(f);
+  }
+  if (!out_dev) {
+    CVCB_TRY(ensure_buffer(L, SLOT_F1, fb, &f));
+    out = static_cast<double *>(f);
+  }
+  CVCB_TRY(launch_tm_full_cvc(L, out, in, a, b, c, g5out));
+  if (!out_dev) CVCB_CUDA(cudaMemcpyAsync(xi, out, fb, cudaMemcpyDeviceToHost, L->stream));
   CVCB_CUDA(cudaStreamSynchronize(L->stream));
   return CVCB_OK;
 }

@@ -259,6 +259,9 @@ enum BufSlot {
 // H in = sum_mu [(1-g_mu) U_mu(x) in(x+mu) + (1+g_mu) U_mu(x-mu)^+ in(x-mu)]
 int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, double b, double c,
                    bool g5out, const int *done_flag);
+// the same on CVC-layout device arrays (16-byte aligned, not overlapping)
+int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a, double b, double c,
+                       bool g5out);
 int launch_g5(cvcb_lattice *L, double2 *f, int nsites);
 int launch_one_pm_imu_inv(cvcb_lattice *L, double2 *f, double sign, int nsites);
 

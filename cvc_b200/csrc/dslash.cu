@@ -139,6 +139,129 @@ int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, d
   return CVCB_OK;
 }
 
+// The same operator on CVC-layout fields (192 contiguous bytes per site), for
+// the entry points that apply it once: no copy into and out of the device
+// layout, which cost two field passes more than the operator itself.  Thread =
+// lexicographic site; a spinor is six 32-byte loads (one whole sector each; V4)
+// or twelve 16-byte ones (fields off a 32-byte boundary).  Same terms in the
+// same order as k_tm_full_f64: the same bits.  A call takes 17 us at 4^3 x 8
+// (25 with the two copies), 29 (44) at 22 x 14 x 10 x 18 and 613 (818) at
+// 32^3 x 64; compulsory traffic there 2.0 GB, 0.31 ms.  Bound by L1: the
+// strided spinor loads keep its data pipe 82 % busy.
+template <bool V4>
+__device__ __forceinline__ Spinor<double> load_spinor_cvc(const double2 *__restrict__ f, int lex) {
+  const double2 *q = f + (size_t)lex * 12;
+  Spinor<double> s;
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    Cx<double> a, b;
+    if (V4) {
+      asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                   : "=d"(a.re), "=d"(a.im), "=d"(b.re), "=d"(b.im)
+                   : "l"(q + 2 * m));
+    } else {
+      const double2 v = __ldg(q + 2 * m), w = __ldg(q + 2 * m + 1);
+      a = cx(v.x, v.y);
+      b = cx(w.x, w.y);
+    }
+    s.c[(2 * m) / 3][(2 * m) % 3] = a;
+    s.c[(2 * m + 1) / 3][(2 * m + 1) % 3] = b;
+  }
+  return s;
+}
+
+template <bool V4>
+__device__ __forceinline__ void store_spinor_cvc(double2 *f, int lex, const Spinor<double> &s) {
+  double2 *q = f + (size_t)lex * 12;
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    const Cx<double> a = s.c[(2 * m) / 3][(2 * m) % 3], b = s.c[(2 * m + 1) / 3][(2 * m + 1) % 3];
+    if (V4) {
+      asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(q + 2 * m), "d"(a.re), "d"(a.im),
+                   "d"(b.re), "d"(b.im)
+                   : "memory");
+    } else {
+      q[2 * m] = make_double2(a.re, a.im);
+      q[2 * m + 1] = make_double2(b.re, b.im);
+    }
+  }
+}
+
+constexpr int kCvcThreads = 128;
+template <bool G5OUT, bool V4>
+__global__ void __launch_bounds__(kCvcThreads, 3)
+    k_tm_full_cvc(double2 *__restrict__ out, const double2 *__restrict__ in,
+                  const double2 *__restrict__ U, Geom g, double a, double b, double c) {
+  const int lex = blockIdx.x * kCvcThreads + threadIdx.x;
+  if (lex >= g.V) return;
+  SiteCoord cd;
+  {
+    const unsigned r0 = fdiv((unsigned)lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
+    cd.lex = lex;
+    cd.z = lex - (int)r0 * g.LZ;
+    cd.y = (int)(r0 - r1 * g.LY);
+    cd.x = (int)(r1 - r2 * g.LX);
+    cd.t = (int)r2;
+  }
+  const int par = (cd.t + cd.x + cd.y + cd.z) & 1;
+  const int self = par * g.Vh + (lex >> 1), qoff = (1 - par) * g.Vh;
+  const size_t V = g.V;
+
+  Spinor<double> acc;
+#pragma unroll
+  for (int sp = 0; sp < 4; ++sp)
+#pragma unroll
+    for (int co = 0; co < 3; ++co) acc.c[sp][co] = cx(0.0, 0.0);
+#pragma unroll
+  for (int mu = 0; mu < 4; ++mu) {
+    {
+      const int j = nb_lex(g, cd, mu, -1);
+      const HalfSpinor<double> h = project(mu, +1, load_spinor_cvc<V4>(in, j));
+      accum_recon(mu, +1, acc, link_dag_mul(load_link64(U, V, mu, qoff + (j >> 1)), h));
+    }
+    {
+      const int j = nb_lex(g, cd, mu, +1);
+      const HalfSpinor<double> h = project(mu, -1, load_spinor_cvc<V4>(in, j));
+      accum_recon(mu, -1, acc, link_mul(load_link64(U, V, mu, self), h));
+    }
+  }
+  const Spinor<double> f = load_spinor_cvc<V4>(in, lex);
+  Spinor<double> r;
+#pragma unroll
+  for (int sp = 0; sp < 4; ++sp) {
+    const double bs = sp < 2 ? b : -b;  // i b g5
+#pragma unroll
+    for (int co = 0; co < 3; ++co) {
+      const Cx<double> v = f.c[sp][co];
+      Cx<double> o;
+      o.re = fma(c, acc.c[sp][co].re, fma(a, v.re, -bs * v.im));
+      o.im = fma(c, acc.c[sp][co].im, fma(a, v.im, bs * v.re));
+      if (G5OUT && sp >= 2) o = cx(-o.re, -o.im);
+      r.c[sp][co] = o;
+    }
+  }
+  store_spinor_cvc<V4>(out, lex, r);
+}
+
+int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a, double b, double c,
+                       bool g5out) {
+  const Geom &g = L->g;
+  const int blocks = (g.V + kCvcThreads - 1) / kCvcThreads;
+  double2 *o = reinterpret_cast<double2 *>(out);
+  const double2 *i = reinterpret_cast<const double2 *>(in);
+  const bool v4 = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 31) == 0;
+  if (g5out && v4)
+    k_tm_full_cvc<true, true><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+  else if (g5out)
+    k_tm_full_cvc<true, false><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+  else if (v4)
+    k_tm_full_cvc<false, true><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+  else
+    k_tm_full_cvc<false, false><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+  CVCB_LAUNCHED(L);
+  return CVCB_OK;
+}
+
 // f = g5 f on the first nsites sites (device layout: spins 2,3 are k = 6..11)
 __global__ void k_g5(double2 *f, Geom g, int nsites_lex) {
   const int lex = blockIdx.x * blockDim.x + threadIdx.x;

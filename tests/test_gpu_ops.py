@@ -132,3 +132,37 @@ def test_errors(cb):
     with pytest.raises(cb.CvcbError):
         cb.Lattice(3, 4, 4, 4)  # odd extent
     lat.close()
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 4, 10), (4, 2, 14, 6)],
+                         ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("where", ["host", "device", "device16", "to_host", "in_place"])
+def test_operator_on_cvc_fields(cb, oracle_mod, dims, where):
+    """The operator on site-major arrays: extents of two (both hops reach the
+    same site), a last block that is not full, fields on 32- and on 16-byte
+    boundaries, mixed memories, and input and output the same array."""
+    torch = pytest.importorskip("torch")
+    bc = (1.0, 0.0, 0.25, 0.5)
+    lat = cb.Lattice(*dims, kappa=0.14, mu=0.03, bc_angle=bc)
+    V = lat.VOLUME
+    g = cb.gauge_random(*dims, 0.3, 4)
+    lat.upload_gauge(g)
+    orc = oracle_mod.Oracle(*dims, 0.14, 0.03, bc)
+    orc.set_gauge(g)
+    phi = seeded(6, 24 * V)
+
+    def dev(off):
+        t = torch.zeros(24 * V + 4, dtype=torch.float64, device="cuda")[off:24 * V + off]
+        t.copy_(torch.from_numpy(phi))
+        torch.cuda.synchronize()
+        return t
+
+    for name, extra in (("Q_phi_tbc", ()), ("Qf5", (-0.02,)), ("Hopping", ())):
+        x = phi.copy() if where == "host" else dev(2 if where == "device16" else 0)
+        y = x if where == "in_place" else np.zeros(24 * V) if where in ("host", "to_host") else \
+            torch.zeros_like(x)
+        torch.cuda.synchronize()
+        getattr(lat, name)(y, x, *extra)
+        got = y if isinstance(y, np.ndarray) else y.cpu().numpy()
+        assert rel_err(got, getattr(orc, name)(phi, *extra)) < 1e-14
+    lat.close()
