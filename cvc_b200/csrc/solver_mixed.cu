@@ -683,8 +683,7 @@ void mailbox(cvcb_lattice *L, int slot, std::vector<double> &out, int n) {
 // ---------------------------------------------------------------------------
 struct LaunchShape {
   int bx = 64, by = 1, nr = 1;  // sites per block, rhs groups per block, rhs per thread
-  int pk = 0;                   // 1: nr == 2 in packed FP32x2 arithmetic (k_eo_hop_x2, k_eo_hop_pt);
-                                // pair-tiled only: 2 k_eo_hop_ptb, 3 and 4 k_eo_hop_ptm
+  int pk = 0;                   // 1: nr == 2 in packed FP32x2 arithmetic (k_eo_hop_x2, k_eo_hop_pt)
 };
 
 // Autotuner results, per process: (V, precision, recon, n) -> launch shape,
@@ -734,7 +733,6 @@ struct Batch {
   // that produces M p
   double *dot_part = nullptr;
   int dot_np = 0;
-  int *err = nullptr;  // set by a stencil whose staged copy did not complete
   int *ru_skip;   // per rhs: 1 = skip in the reliable update
   int *rst_skip;  // per rhs: 0 = restart the direction from the residual
   BatchRed br;
@@ -771,7 +769,6 @@ struct Batch {
       a.dot_np = dot_parts();
       dot_np = a.dot_np;
     }
-    a.err = err;
     // FP64 sweeps of a reduced-precision solve (reliable updates) have their
     // own tuned shape; FP64 kernels keep one rhs per thread (register budget).
     LaunchShape sh = sizeof(typename AF::R) == 8 && sizeof(typename SF::R) != 8 ? shape64 : shape;
@@ -855,8 +852,7 @@ struct Batch {
       dot_np = a.dot_np;
       a.rup = rs;
       a.alpha = S.alpha;
-      a.err = err;
-      Rec rec{};
+        Rec rec{};
       if (prof_rec) {
         CVCB_CUDA(cudaEventCreate(&rec.a));
         CVCB_CUDA(cudaEventCreate(&rec.b));
@@ -892,52 +888,18 @@ struct Batch {
     return sizeof(typename SF::R) == 4 && shape.pk >= 1 && shape.bx % 32 == 0;
   }
   // partial sums per rhs of the fused norms: one per warp of the site blocks
-  // (one per 32-site tile for the bulk-staged stencil)
   int dot_parts() const {
-    if (shape.pk == 2) return g.Vh / kTile;
     return ((g.Vh + shape.bx - 1) / shape.bx) * (shape.bx / 32);
   }
 
-  // Pair-tiled stencil launch: pk 2 = bulk-staged t and x neighbours
-  // (k_eo_hop_ptb, whole-tile lattices only), pk 3, 4 = accumulator in
-  // tensor memory (k_eo_hop_ptm, 24 warps per SM / next direction's loads in
-  // flight), else plain loads (k_eo_hop_pt)
+  // Pair-tiled stencil launch
   template <class LL, bool G5IN, bool G5HOP, bool AUX, bool RUPD>
   int launch_pt(const HopArgs<P32, LL> &a, const LaunchShape &sh) {
     const int groups = (n + 1) / 2;
-    if (sh.pk == 2) {
-      if (!bulk_stencil_ok(g) || !a.err) {
-        set_error("bulk-staged stencil needs LY*LZ/2 a multiple of 32");
-        return CVCB_ERR_ARG;
-      }
-      auto kern = k_eo_hop_ptb<LL, G5IN, G5HOP, AUX, RUPD>;
-      static std::atomic<unsigned long long> attr_set{0};  // per instantiation, bit per device
-      const unsigned long long bit = 1ull << (L->device & 63);
-      if (!(attr_set.load() & bit)) {
-        CVCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kBulkSmem));
-        attr_set.fetch_or(bit);
-      }
-      const int tiles = g.Vh / kTile;
-      dim3 grid(groups, std::min((tiles + kBulkWarps - 1) / kBulkWarps, 65535));
-      kern<<<grid, kBulkWarps * 32, kBulkSmem, L->stream>>>(a);
-    } else {
-      const int by = std::min(sh.by, groups);
-      const int site_blocks = (g.Vh + sh.bx - 1) / sh.bx;
-      dim3 block(sh.bx, by), grid((groups + by - 1) / by, std::min(site_blocks, 65535));
-      if (sh.pk == 3 || sh.pk == 4) {  // accumulator in tensor memory: 128 sites, one pair per block
-        if (sh.bx != kTmemThreads || sh.by != 1) {
-          set_error("tensor-memory stencil needs 128 sites and one rhs pair per block");
-          return CVCB_ERR_ARG;
-        }
-        if (sh.pk == 3)
-          k_eo_hop_ptm<LL, G5IN, G5HOP, AUX, RUPD, false><<<grid, kTmemThreads, 0, L->stream>>>(a);
-        else
-          k_eo_hop_ptm<LL, G5IN, G5HOP, AUX, RUPD, true><<<grid, kTmemThreads, 0, L->stream>>>(a);
-      } else {
-        k_eo_hop_pt<LL, G5IN, G5HOP, AUX, RUPD><<<grid, block, 0, L->stream>>>(a);
-      }
-    }
+    const int by = std::min(sh.by, groups);
+    const int site_blocks = (g.Vh + sh.bx - 1) / sh.bx;
+    dim3 block(sh.bx, by), grid((groups + by - 1) / by, std::min(site_blocks, 65535));
+    k_eo_hop_pt<LL, G5IN, G5HOP, AUX, RUPD><<<grid, block, 0, L->stream>>>(a);
     CVCB_LAUNCHED(L);
     return CVCB_OK;
   }
@@ -1163,7 +1125,7 @@ int setup_batch(cvcb_lattice *L, Batch<SF, XF, LF> &B, int n, bool with_fp64 = t
                       rnd(sizeof(unsigned) * kMaxBatch);
   const size_t dotb = sizeof(double) * (size_t)n * (g.Vh / 32 + 64);
   const size_t total = 5 * rnd(f64) + 6 * (rnd(sl) + rnd(nrm)) + rnd(xsl) + rnd(nrm) + scal + part +
-                       rnd(dotb) + rnd(sizeof(int));
+                       rnd(dotb);
   void *mem;
   CVCB_TRY(ensure_buffer(L, SLOT_MIX0, total, &mem));
   char *p = static_cast<char *>(mem);
@@ -1204,8 +1166,6 @@ int setup_batch(cvcb_lattice *L, Batch<SF, XF, LF> &B, int n, bool with_fp64 = t
   B.br.partials = (double *)take(sizeof(double) * kMaxRedBlocks * kMaxBatch * 2);
   B.br.counters = (unsigned *)take(sizeof(unsigned) * kMaxBatch);
   B.dot_part = (double *)take(dotb);
-  B.err = (int *)take(sizeof(int));
-  CVCB_CUDA(cudaMemsetAsync(B.err, 0, sizeof(int), L->stream));
   CVCB_CUDA(cudaMemsetAsync(B.br.counters, 0, sizeof(unsigned) * kMaxBatch, L->stream));
   CVCB_CUDA(cudaMemsetAsync(B.S.done, 0, sizeof(int) * kMaxBatch, L->stream));
   CVCB_CUDA(cudaMemsetAsync(B.ru_skip, 0, sizeof(int) * kMaxBatch, L->stream));
@@ -1263,14 +1223,7 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
         f.bx * f.by <= kHopMaxThreads) {
       if (nf < 4 || f.nr != 2) f.pk = 0;
       if (sizeof(typename SF::R) == 8) f.nr = 1, f.pk = 0;
-      if (pairs) {  // pair-tiled fields: one rhs pair per thread; 4th field 2 = bulk-staged
-        f.nr = 2;
-        f.pk = (nf >= 4 && f.pk == 2 && bulk_stencil_ok(L->g)) ? 2
-               : (nf >= 4 && (f.pk == 3 || f.pk == 4))           ? f.pk
-                                                                 : 1;
-        if (f.pk == 2) f.bx = kBulkWarps * 32, f.by = 1;
-        if (f.pk >= 3) f.bx = kTmemThreads, f.by = 1;
-      }
+      if (pairs) f.nr = 2, f.pk = 1;  // pair-tiled fields: one rhs pair per thread
       B.shape = f;
       g_tuned_shape[key] = f;
       return CVCB_OK;
@@ -1308,28 +1261,6 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
         best = B.shape;
       }
     }
-  if (pairs) {  // the tensor-memory accumulator: one fixed block shape, two register budgets
-    for (int pk : {3, 4}) {
-      B.shape = LaunchShape{kTmemThreads, 1, 2, pk};
-      float ms;
-      if (time_ms(L, [&] { return B.normal_op_sloppy(B.Ap, B.p, nullptr); }, 3, &ms) != CVCB_OK) {
-        cudaGetLastError();
-      } else if (ms < best_ms) {
-        best_ms = ms;
-        best = B.shape;
-      }
-    }
-  }
-  if (pairs && bulk_stencil_ok(L->g)) {  // the bulk-staged stencil: one fixed block shape
-    B.shape = LaunchShape{kBulkWarps * 32, 1, 2, 2};
-    float ms;
-    if (time_ms(L, [&] { return B.normal_op_sloppy(B.Ap, B.p, nullptr); }, 3, &ms) != CVCB_OK) {
-      cudaGetLastError();
-    } else if (ms < best_ms) {
-      best_ms = ms;
-      best = B.shape;
-    }
-  }
   B.shape = best;
   g_tuned_shape[key] = best;
   return CVCB_OK;
@@ -1645,13 +1576,6 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
     const double rel = hb2[i] > 0 ? std::sqrt(rhat2[i] / hb2[i]) : 0.0;
     worst = std::max(worst, rel);
     if (rel <= P->tol) ++nconv;
-  }
-  int staged_err = 0;
-  CVCB_CUDA(cudaMemcpyAsync(&staged_err, B.err, sizeof(int), cudaMemcpyDeviceToHost, L->stream));
-  CVCB_CUDA(cudaStreamSynchronize(L->stream));
-  if (staged_err) {
-    set_error("a staged neighbour copy of the stencil did not complete in time");
-    return CVCB_ERR_CUDA;
   }
   st->iterations += std::accumulate(iters.begin(), iters.end(), 0);
   st->reliable_updates += nru;
@@ -2043,7 +1967,7 @@ int cvcb_tuned_shape(cvcb_lattice *L, int precision, int link_recon, int nrhs, i
   *sites_per_block = s.bx;
   *rows_per_block = s.by;
   *rhs_per_thread = s.nr;
-  *variant = pairs ? (s.pk >= 3 ? 1 + s.pk : s.pk == 2 ? 6 : 3) : s.pk ? 2 : (s.by > 1 && s.nr == 1) ? 1 : 0;
+  *variant = pairs ? 3 : s.pk ? 2 : (s.by > 1 && s.nr == 1) ? 1 : 0;
   return CVCB_OK;
 }
 
