@@ -252,6 +252,14 @@ struct EoGeom {
   int p;  // output parity
 };
 
+// What the last block of a sweep does with the sums of dot_part (k_eo_hop_sp):
+// kind 1: alpha = rr / sum, 2: beta = sum / rr and rr = sum, 0: nothing.
+struct DotFinish {
+  int kind;
+  unsigned *counters;  // per rhs pair, zero between launches
+  double *rr, *pAp, *alpha, *beta;
+};
+
 // Per-call arguments of the stencil kernel.
 template <class SF, class LF>
 struct HopArgs {
@@ -273,6 +281,7 @@ struct HopArgs {
   // |r|^2)
   SF rup;
   const double *alpha;
+  DotFinish fin;
 };
 
 // |a|^2 of one site, accumulated in FP64

@@ -21,6 +21,7 @@
 #pragma once
 
 #include "eo_kernels.cuh"
+#include "reduce.cuh"
 
 namespace cvcb {
 
@@ -344,6 +345,209 @@ __global__ void __launch_bounds__(kHopMaxThreads, 2) k_eo_hop_pt(HopArgs<P32, LF
         if (has_b) A.dot_part[(size_t)(ra + 1) * A.dot_np + w] = db;
       }
     }
+  }
+}
+
+// ---- the same sweep with a site's eight directions on eight warps -----------
+// One thread per site and pair goes through the directions one after the
+// other, eight load latencies in a row, and on a small lattice the GPU has
+// nothing else to do meanwhile.  Here block = one 32-site tile of one pair,
+// warp d = direction (z-, z+, y-, y+, x-, x+, t-, t+, the order of
+// hop_pair_dir): every warp loads one neighbour, leaves its transported half
+// spinors in shared memory, and warps 0..2 sum the colours 0..2 over the
+// directions and run the epilogue.  The sums run in the order of k_eo_hop_pt:
+// the same field values to the last bit.
+constexpr int kSplitThreads = 256;
+
+template <int MU, bool DAG, class LF>
+__device__ __forceinline__ void split_dir(float4 (*sh)[kTile], const HopArgs<P32, LF> &A,
+                                          const SiteCoord &cd, int pr, int self, int qoff,
+                                          bool g5in, int lane) {
+  const int j = nb_lex(A.eg.g, cd, MU, DAG ? -1 : +1) >> 1;
+  const Link<float> W = A.links.load(MU, DAG ? qoff + j : self);
+  const SpinorPair f = A.in.load_pair(pr, j);
+  constexpr int S = DAG ? +1 : -1;
+  const HalfPair h = g5in ? project_pair<MU, -S>(f) : project_pair<MU, S>(f);
+  const HalfPair u = link_mul_pair<DAG>(W, h);
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh[3 * b + c][lane] = f4_of(u.c[b][c]);
+}
+
+// a (spin s of one colour) += (1 + S g_mu)-reconstruction of u (spins 0, 1 of
+// the colour): accum_recon_pair, one component
+template <int MU, int S>
+__device__ __forceinline__ void recon_add(CP (&a)[4], const CP (&u)[2]) {
+  auto add = [](CP &x, const CP &v, bool plus) {
+    x.re = plus ? add2(x.re, v.re) : sub2(x.re, v.re);
+    x.im = plus ? add2(x.im, v.im) : sub2(x.im, v.im);
+  };
+  auto add_i = [](CP &x, const CP &v, bool plus) {  // x += +-i v
+    x.re = plus ? sub2(x.re, v.im) : add2(x.re, v.im);
+    x.im = plus ? add2(x.im, v.re) : sub2(x.im, v.re);
+  };
+  add(a[0], u[0], true);
+  add(a[1], u[1], true);
+  if (MU == 0) {  // r2 = -S u0, r3 = -S u1
+    add(a[2], u[0], S < 0);
+    add(a[3], u[1], S < 0);
+  } else if (MU == 1) {  // r2 = S i u1, r3 = S i u0
+    add_i(a[2], u[1], S > 0);
+    add_i(a[3], u[0], S > 0);
+  } else if (MU == 2) {  // r2 = S u1, r3 = -S u0
+    add(a[2], u[1], S > 0);
+    add(a[3], u[0], S < 0);
+  } else {  // r2 = S i u0, r3 = -S i u1
+    add_i(a[2], u[0], S > 0);
+    add_i(a[3], u[1], S < 0);
+  }
+}
+
+// alpha or beta of right-hand side r from the sum t of a sweep's partials
+__device__ __forceinline__ void dot_epilogue(const DotFinish &f, int r, double t) {
+  if (f.kind == 1) {
+    f.pAp[r] = t;
+    // M^+ M is positive definite; a non-positive <p, M^+ M p> only comes from
+    // rounding at the end of convergence: take no step and let the host's
+    // reliable update refresh the residual.
+    f.alpha[r] = (t > 0 && isfinite(t)) ? f.rr[r] / t : 0.0;
+  } else {
+    f.beta[r] = t / f.rr[r];
+    f.rr[r] = t;
+  }
+}
+
+static_assert(kSplitThreads == kRedThreads, "the last block reduces with block_sum");
+template <class LF, bool G5IN, bool G5HOP, bool AUX, bool RUPD = false>
+__global__ void __launch_bounds__(kSplitThreads) k_eo_hop_sp(const __grid_constant__ HopArgs<P32, LF> A) {
+  __shared__ float4 sh[8][6][kTile];
+  __shared__ double2 sn[3];
+  const int pr = blockIdx.x, ra = 2 * pr;
+  const bool act_a = !(A.done && A.done[ra]);
+  const bool has_b = ra + 1 < A.nrhs;
+  const bool act_b = has_b && !(A.done && A.done[ra + 1]);
+  if (!act_a && !act_b) return;
+  const Geom &g = A.eg.g;
+  const int p = A.eg.p, qoff = (1 - p) * g.Vh;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles = (g.Vh + kTile - 1) / kTile;
+  for (int tile = blockIdx.y; tile < tiles; tile += gridDim.y) {
+    const int i = tile * kTile + lane;
+    const bool valid = i < g.Vh;
+    // the epilogue's own inputs are under way while the directions arrive
+    float4 ax[4], rx[4];
+    if (valid && warp < 3) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        if (AUX) ax[s] = __ldg(A.aux.at(pr, i) + P32::comp(3 * s + warp));
+        if (RUPD) rx[s] = __ldg(A.rup.at(pr, i) + P32::comp(3 * s + warp));
+      }
+    }
+    if (valid) {
+      const SiteCoord cd = site_coord(g, p, i);
+      const int self = p * g.Vh + i;
+      switch (warp) {
+        case 0: split_dir<3, true>(sh[0], A, cd, pr, self, qoff, G5IN, lane); break;
+        case 1: split_dir<3, false>(sh[1], A, cd, pr, self, qoff, G5IN, lane); break;
+        case 2: split_dir<2, true>(sh[2], A, cd, pr, self, qoff, G5IN, lane); break;
+        case 3: split_dir<2, false>(sh[3], A, cd, pr, self, qoff, G5IN, lane); break;
+        case 4: split_dir<1, true>(sh[4], A, cd, pr, self, qoff, G5IN, lane); break;
+        case 5: split_dir<1, false>(sh[5], A, cd, pr, self, qoff, G5IN, lane); break;
+        case 6: split_dir<0, true>(sh[6], A, cd, pr, self, qoff, G5IN, lane); break;
+        default: split_dir<0, false>(sh[7], A, cd, pr, self, qoff, G5IN, lane); break;
+      }
+    }
+    __syncthreads();
+    if (warp < 3) {
+      double2 n2 = make_double2(0.0, 0.0);
+      if (valid) {
+        CP acc[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) acc[s].re = acc[s].im = make_float2(0.f, 0.f);
+        auto take = [&](int d, CP (&u)[2]) {
+          u[0] = cp_of(sh[d][warp][lane]);
+          u[1] = cp_of(sh[d][3 + warp][lane]);
+        };
+        CP u[2];
+        take(0, u), recon_add<3, +1>(acc, u);
+        take(1, u), recon_add<3, -1>(acc, u);
+        take(2, u), recon_add<2, +1>(acc, u);
+        take(3, u), recon_add<2, -1>(acc, u);
+        take(4, u), recon_add<1, +1>(acc, u);
+        take(5, u), recon_add<1, -1>(acc, u);
+        take(6, u), recon_add<0, +1>(acc, u);
+        take(7, u), recon_add<0, -1>(acc, u);
+        float4 *dst = RUPD ? A.rup.at(pr, i) : A.out.at(pr, i);
+        const float2 na = RUPD ? make_float2(-(float)A.alpha[ra], has_b ? -(float)A.alpha[ra + 1] : 0.f)
+                               : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const float g5 = s < 2 ? 1.f : -1.f, gh = G5HOP ? g5 : 1.f;
+          const float a1 = (float)(A.c * A.d1a) * gh, b1 = (float)(A.c * A.d1b) * g5 * gh;
+          const float a2 = (float)A.d2a, b2 = (float)A.d2b * g5;
+          CP o;  // diag_pair, one component
+          o.re = __ffma2_rn(bc(-b1), acc[s].im, __fmul2_rn(bc(a1), acc[s].re));
+          o.im = __ffma2_rn(bc(b1), acc[s].re, __fmul2_rn(bc(a1), acc[s].im));
+          if (AUX) {
+            const CP x = cp_of(ax[s]);
+            o.re = __ffma2_rn(bc(-b2), x.im, __ffma2_rn(bc(a2), x.re, o.re));
+            o.im = __ffma2_rn(bc(b2), x.re, __ffma2_rn(bc(a2), x.im, o.im));
+          }
+          if (RUPD) {
+            CP rv = cp_of(rx[s]);
+            rv.re = __ffma2_rn(na, o.re, rv.re);
+            rv.im = __ffma2_rn(na, o.im, rv.im);
+            o = rv;
+          }
+          n2.x = fma((double)o.re.x, (double)o.re.x, fma((double)o.im.x, (double)o.im.x, n2.x));
+          n2.y = fma((double)o.re.y, (double)o.re.y, fma((double)o.im.y, (double)o.im.y, n2.y));
+          float4 *q = dst + P32::comp(3 * s + warp);
+          if (act_a && act_b) {
+            *q = f4_of(o);
+          } else {
+            float *f = reinterpret_cast<float *>(q) + (act_a ? 0 : 1);
+            f[0] = act_a ? o.re.x : o.re.y;
+            f[2] = act_a ? o.im.x : o.im.y;
+          }
+        }
+      }
+      if (A.dot_part) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          n2.x += __shfl_down_sync(0xffffffffu, n2.x, o);
+          n2.y += __shfl_down_sync(0xffffffffu, n2.y, o);
+        }
+        if (lane == 0) sn[warp] = n2;
+      }
+    }
+    __syncthreads();  // also: the next tile overwrites sh
+    if (A.dot_part && threadIdx.x == 0) {
+      A.dot_part[(size_t)ra * A.dot_np + tile] = sn[0].x + sn[1].x + sn[2].x;
+      if (has_b) A.dot_part[(size_t)(ra + 1) * A.dot_np + tile] = sn[0].y + sn[1].y + sn[2].y;
+    }
+  }
+  if (!A.dot_part || !A.fin.kind) return;
+  // the pair's last block sums the partials, in k_dot_finish's order
+  __shared__ bool last;
+  __shared__ double sr[2][kRedThreads / 32];
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(A.fin.counters + pr, 1u) == gridDim.y - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double v[2] = {0.0, 0.0};
+  for (int k = threadIdx.x; k < A.dot_np; k += kRedThreads) {
+    v[0] += __ldcg(A.dot_part + (size_t)ra * A.dot_np + k);
+    if (has_b) v[1] += __ldcg(A.dot_part + (size_t)(ra + 1) * A.dot_np + k);
+  }
+  block_sum<2>(v, sr);
+  if (threadIdx.x == 0) {
+    A.fin.counters[pr] = 0;
+    if (act_a) dot_epilogue(A.fin, ra, v[0]);
+    if (act_b) dot_epilogue(A.fin, ra + 1, v[1]);
   }
 }
 

@@ -130,11 +130,7 @@ struct RedPAp {
 struct EpiAlphaB {
   Scal S;
   __device__ void operator()(int r, double t) const {
-    S.pAp[r] = t;
-    // M^+ M is positive definite; a non-positive <p, M^+ M p> only comes from
-    // rounding at the end of convergence: take no step and let the host's
-    // reliable update refresh the residual.
-    S.alpha[r] = (t > 0 && isfinite(t)) ? S.rr[r] / t : 0.0;
+    dot_epilogue(DotFinish{1, nullptr, S.rr, S.pAp, S.alpha, S.beta}, r, t);
   }
 };
 
@@ -178,8 +174,7 @@ struct RedUpdate {
 struct EpiBetaB {
   Scal S;
   __device__ void operator()(int r, double t) const {
-    S.beta[r] = t / S.rr[r];
-    S.rr[r] = t;
+    dot_epilogue(DotFinish{2, nullptr, S.rr, S.pAp, S.alpha, S.beta}, r, t);
   }
 };
 
@@ -208,33 +203,42 @@ __global__ void k_p_upd(SF p, SF rs, XF xs, Scal S, int nsites, int nrhs) {
   p.store(r, s, pv);
 }
 
-// Pair-tiled form of the CG vector update (thread = site x rhs pair, packed
-// FP32x2 arithmetic; an inactive right-hand side keeps its values).  The
+// Pair-tiled form of the CG vector update (thread = 32 bytes of a site and rhs
+// pair, packed FP32x2 arithmetic; an inactive right-hand side keeps its values).  The
 // residual update r -= alpha A p runs inside the last stencil sweep.
 // x_s += alpha p; p = r_s + beta p
-__global__ void k_p_upd_pt(P32 p, P32 rs, P32 xs, Scal S, int nsites, int nrhs) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ra = 2 * blockIdx.y;
+constexpr int kUpdTiles = 2;  // tiles per block: 6 warps each, one component pair per warp
+__global__ void __launch_bounds__(kUpdTiles * 192)
+    k_p_upd_pt(P32 p, P32 rs, P32 xs, Scal S, int nsites, int nrhs) {
+  const int tile = blockIdx.x * kUpdTiles + threadIdx.x / 192, m = threadIdx.x % 192 / 32;
+  const int s = tile * kTile + (threadIdx.x & 31), pr = blockIdx.y;
+  const int ra = 2 * pr;
   if (s >= nsites) return;
   const bool act_a = !S.done[ra];
   const bool act_b = ra + 1 < nrhs && !S.done[ra + 1];
   if (!act_a && !act_b) return;
-  const float2 a = make_float2((float)S.alpha[ra], act_b ? (float)S.alpha[ra + 1] : 0.f);
-  const float2 b = make_float2((float)S.beta[ra], act_b ? (float)S.beta[ra + 1] : 0.f);
-  const SpinorPair rv = rs.load_pair(blockIdx.y, s);
-  SpinorPair pv = p.load_pair(blockIdx.y, s);
-  SpinorPair xv = xs.load_pair(blockIdx.y, s);
+  const float2 av = make_float2((float)S.alpha[ra], act_b ? (float)S.alpha[ra + 1] : 0.f);
+  const float2 bv = make_float2((float)S.beta[ra], act_b ? (float)S.beta[ra + 1] : 0.f);
+  const size_t off = m * 2 * kTile;
+  float4 r[2], q[2], x[2];
+  ldg_v8(rs.at(pr, s) + off, r[0], r[1]);
+  ldg_v8(p.at(pr, s) + off, q[0], q[1]);
+  ldg_v8(xs.at(pr, s) + off, x[0], x[1]);
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      xv.c[k][c].re = __ffma2_rn(a, pv.c[k][c].re, xv.c[k][c].re);
-      xv.c[k][c].im = __ffma2_rn(a, pv.c[k][c].im, xv.c[k][c].im);
-      pv.c[k][c].re = __ffma2_rn(b, pv.c[k][c].re, rv.c[k][c].re);
-      pv.c[k][c].im = __ffma2_rn(b, pv.c[k][c].im, rv.c[k][c].im);
-    }
-  store_active(xs, blockIdx.y, s, xv, act_a, act_b);
-  store_active(p, blockIdx.y, s, pv, act_a, act_b);
+  for (int h = 0; h < 2; ++h) {
+    const CP rc = cp_of(r[h]), pc = cp_of(q[h]), xc = cp_of(x[h]);
+    CP xn, pn;
+    xn.re = __ffma2_rn(av, pc.re, xc.re);
+    xn.im = __ffma2_rn(av, pc.im, xc.im);
+    pn.re = __ffma2_rn(bv, pc.re, rc.re);
+    pn.im = __ffma2_rn(bv, pc.im, rc.im);
+    if (!act_a) xn.re.x = xc.re.x, xn.im.x = xc.im.x, pn.re.x = pc.re.x, pn.im.x = pc.im.x;
+    if (!act_b) xn.re.y = xc.re.y, xn.im.y = xc.im.y, pn.re.y = pc.re.y, pn.im.y = pc.im.y;
+    x[h] = f4_of(xn);
+    q[h] = f4_of(pn);
+  }
+  stg_v8(xs.at(pr, s) + off, x[0], x[1]);
+  stg_v8(p.at(pr, s) + off, q[0], q[1]);
 }
 
 // Pair-tiled forms of the reliable-update kernels below: thread = site x rhs
@@ -684,6 +688,7 @@ void mailbox(cvcb_lattice *L, int slot, std::vector<double> &out, int n) {
 struct LaunchShape {
   int bx = 64, by = 1, nr = 1;  // sites per block, rhs groups per block, rhs per thread
   int pk = 0;                   // 1: nr == 2 in packed FP32x2 arithmetic (k_eo_hop_x2, k_eo_hop_pt)
+                                // 2: pair-tiled, a site's directions on eight warps (k_eo_hop_sp)
 };
 
 // Autotuner results, per process: (V, precision, recon, n) -> launch shape,
@@ -758,8 +763,9 @@ struct Batch {
   // writes per-warp partials of |out|^2 (dot_np per rhs).
   template <class AF, class LL, bool G5IN, bool G5HOP, bool AUX>
   int hop(AF out, AF in, AF aux, LL lk, int parity, const int *done, double d1a, double d1b,
-          double d2a, double d2b, double c, double *dot_part = nullptr) {
+          double d2a, double d2b, double c, double *dot_part = nullptr, bool finish = false) {
     HopArgs<AF, LL> a{out, in, aux, lk, EoGeom{g, parity}, n, done, d1a, d1b, d2a, d2b, c};
+    if (finish) a.fin = dot_finish(1);
     if (dot_part) {
       if (!dot_fusable()) {
         set_error("fused norm needs the packed stencil with warp-aligned blocks");
@@ -852,6 +858,7 @@ struct Batch {
       dot_np = a.dot_np;
       a.rup = rs;
       a.alpha = S.alpha;
+      if (finishes_dots()) a.fin = dot_finish(2);
         Rec rec{};
       if (prof_rec) {
         CVCB_CUDA(cudaEventCreate(&rec.a));
@@ -887,6 +894,14 @@ struct Batch {
   bool dot_fusable() const {
     return sizeof(typename SF::R) == 4 && shape.pk >= 1 && shape.bx % 32 == 0;
   }
+  // whether the sweep itself forms alpha and beta from its partials: the
+  // kernel for small lattices, where a launch more counts (2.2 us of about
+  // 20 per iteration at 8^3x16); elsewhere k_dot_finish sums them with one
+  // block per rhs, 6 us of 1.4 ms per iteration at 24^3x48 and 12 rhs
+  bool finishes_dots() const { return std::is_same<SF, P32>::value && shape.pk == 2; }
+  DotFinish dot_finish(int kind) const {
+    return DotFinish{kind, br.counters, S.rr, S.pAp, S.alpha, S.beta};
+  }
   // partial sums per rhs of the fused norms: one per warp of the site blocks
   int dot_parts() const {
     return ((g.Vh + shape.bx - 1) / shape.bx) * (shape.bx / 32);
@@ -896,6 +911,12 @@ struct Batch {
   template <class LL, bool G5IN, bool G5HOP, bool AUX, bool RUPD>
   int launch_pt(const HopArgs<P32, LL> &a, const LaunchShape &sh) {
     const int groups = (n + 1) / 2;
+    if (sh.pk == 2) {
+      dim3 grid(groups, std::min((g.Vh + kTile - 1) / kTile, 65535));
+      k_eo_hop_sp<LL, G5IN, G5HOP, AUX, RUPD><<<grid, kSplitThreads, 0, L->stream>>>(a);
+      CVCB_LAUNCHED(L);
+      return CVCB_OK;
+    }
     const int by = std::min(sh.by, groups);
     const int site_blocks = (g.Vh + sh.bx - 1) / sh.bx;
     dim3 block(sh.bx, by), grid((groups + by - 1) / by, std::min(site_blocks, 65535));
@@ -933,14 +954,19 @@ struct Batch {
       ainv(-mu, ja, jb);
       CVCB_TRY((hop<SF, LF, false, false, false>(te, p, p, links, 0, S.done, ia, ib, 0, 0, -0.5)));
       CVCB_TRY((hop<SF, LF, false, false, true>(yo, te, p, links, 1, S.done, 1, 0, ka(), mu, 0.5,
-                                                dot_part)));
-      k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, dot_np, EpiAlphaB{S}, S.done);
-      CVCB_LAUNCHED(L);
+                                                dot_part, finishes_dots())));
+      if (!finishes_dots()) {
+        k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, dot_np, EpiAlphaB{S}, S.done);
+        CVCB_LAUNCHED(L);
+      }
       CVCB_TRY((hop<SF, LF, true, false, false>(te2, yo, yo, links, 0, S.done, ja, jb, 0, 0, -0.5)));
       CVCB_TRY(hop_rupd(te2, yo, ka(), -mu));
-      k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, dot_np, EpiBetaB{S}, S.done);
-      CVCB_LAUNCHED(L);
-      k_p_upd_pt<<<dim3((g.Vh + 127) / 128, np), 128, 0, L->stream>>>(p, rs, xs, S, g.Vh, n);
+      if (!finishes_dots()) {
+        k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, dot_np, EpiBetaB{S}, S.done);
+        CVCB_LAUNCHED(L);
+      }
+      const int ub = ((g.Vh + kTile - 1) / kTile + kUpdTiles - 1) / kUpdTiles;
+      k_p_upd_pt<<<dim3(ub, np), kUpdTiles * 192, 0, L->stream>>>(p, rs, xs, S, g.Vh, n);
       CVCB_LAUNCHED(L);
       return CVCB_OK;
     }
@@ -1223,7 +1249,11 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
         f.bx * f.by <= kHopMaxThreads) {
       if (nf < 4 || f.nr != 2) f.pk = 0;
       if (sizeof(typename SF::R) == 8) f.nr = 1, f.pk = 0;
-      if (pairs) f.nr = 2, f.pk = 1;  // pair-tiled fields: one rhs pair per thread
+      if (pairs) {  // one rhs pair per thread; 4th field 2: directions on warps
+        f.nr = 2;
+        f.pk = nf >= 4 && f.pk == 2 ? 2 : 1;
+        if (f.pk == 2) f.bx = kTile, f.by = 1;
+      }
       B.shape = f;
       g_tuned_shape[key] = f;
       return CVCB_OK;
@@ -1261,6 +1291,14 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
         best = B.shape;
       }
     }
+  if (pairs) {  // a site's directions on eight warps
+    B.shape = LaunchShape{kTile, 1, 2, 2};
+    float ms;
+    if (time_ms(L, [&] { return B.normal_op_sloppy(B.Ap, B.p, nullptr); }, 3, &ms) != CVCB_OK)
+      cudaGetLastError();
+    else if (ms < best_ms)
+      best = B.shape;
+  }
   B.shape = best;
   g_tuned_shape[key] = best;
   return CVCB_OK;
@@ -1967,7 +2005,7 @@ int cvcb_tuned_shape(cvcb_lattice *L, int precision, int link_recon, int nrhs, i
   *sites_per_block = s.bx;
   *rows_per_block = s.by;
   *rhs_per_thread = s.nr;
-  *variant = pairs ? 3 : s.pk ? 2 : (s.by > 1 && s.nr == 1) ? 1 : 0;
+  *variant = pairs ? (s.pk == 2 ? 4 : 3) : s.pk ? 2 : (s.by > 1 && s.nr == 1) ? 1 : 0;
   return CVCB_OK;
 }
 

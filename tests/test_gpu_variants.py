@@ -71,3 +71,57 @@ def test_stencil_variants_agree(prec):
         assert r["res"] <= 1e-10 and r["chk"] <= 1e-10, (v, r)
         assert abs(r["iters"] - base["iters"]) <= 0.1 * base["iters"], (v, r, base)
         assert abs(r["x4"] - base["x4"]) <= 1e-8 * base["x4"], (v, r, base)
+
+
+SPLIT_CHILD = r"""
+import sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+sys.path.insert(0, sys.argv[1] + "/tests")
+import cvc_b200 as cb
+from conftest import seeded
+dims = tuple(int(v) for v in sys.argv[3].split("x"))
+lat = cb.Lattice(*dims, kappa=0.14, mu=0.02, bc_angle=(1.0, 0.0, 0.5, 0.0))
+lat.upload_gauge(cb.gauge_random(*dims, 0.3, 3))
+V = lat.VOLUME
+out = {}
+for recon in (12, 18):
+    for n in (1, 3):
+        ins = [seeded(10 + i, 24 * V) for i in range(n)]
+        outs = [np.zeros(24 * V) for _ in range(n)]
+        lat.sloppy_normal_op(ins, outs, cb.PREC_SINGLE, recon, 1)
+        out["op%d_%d" % (recon, n)] = np.array(outs)
+        p = cb.solver_defaults()
+        p.link_recon, p.block_rhs = recon, n
+        xs = [np.zeros(24 * V) for _ in range(n)]
+        st = lat.solve(xs, ins, p)
+        assert st.converged == n and st.max_true_res <= 1e-10
+        out["x%d_%d" % (recon, n)] = np.array(xs)
+        out["it%d_%d" % (recon, n)] = np.array([st.iterations])
+np.savez(sys.argv[2], **out)
+"""
+
+
+@pytest.mark.parametrize("dims", ["2x2x2x2", "2x2x6x10", "6x4x2x14"])
+def test_directions_on_warps_same_bits(tmp_path, dims):
+    """The kernel with a site's directions on eight warps against the one with
+    a thread per site: the operator to the last bit, the solves to their 1e-10
+    residual (the norms sum in another order) and iteration count, on half
+    volumes below and off whole tiles of 32, for lone and paired rhs."""
+    import numpy as np
+    got = []
+    for shape in ("64,1,2,1", "32,1,2,2"):
+        f = tmp_path / (shape.replace(",", "_") + ".npz")
+        out = subprocess.run([sys.executable, "-c", SPLIT_CHILD, str(ROOT), str(f), dims],
+                             env=dict(os.environ, CVCB_SHAPE=shape, CVCB_PAIRS="1"),
+                             capture_output=True, text=True, timeout=600)
+        assert out.returncode == 0, out.stderr[-2000:]
+        got.append(np.load(f))
+    a, b = got
+    for k in a.files:
+        if k.startswith("op"):
+            assert np.array_equal(a[k], b[k]), k
+        elif k.startswith("it"):
+            assert abs(int(a[k][0]) - int(b[k][0])) <= 3 + 0.1 * a[k][0], k
+        else:
+            assert np.max(np.abs(a[k] - b[k])) <= 1e-8 * np.max(np.abs(a[k])), k
