@@ -62,6 +62,7 @@ __device__ __forceinline__ void stg_v8(float4 *q, const float4 &a, const float4 
 // (a warp: 1 KB contiguous), six per site and rhs pair.
 struct P32 {
   using R = float;
+  static constexpr bool kScaled = false;  // no scale per site
   float4 *p;
   size_t pstride;  // float4 per pair (tiles x 12 x 32)
   __device__ __forceinline__ static constexpr int comp(int k) { return (k >> 1) * (2 * kTile) + (k & 1); }
@@ -80,6 +81,9 @@ struct P32 {
       s.c[(2 * m + 1) / 3][(2 * m + 1) % 3] = cp_of(b);
     }
     return s;
+  }
+  __device__ __forceinline__ SpinorPair load_pair_raw(int pr, int j, float2 &) const {
+    return load_pair(pr, j);
   }
   __device__ __forceinline__ void store_pair(int pr, int j, const SpinorPair &s) const {
     float4 *q = at(pr, j);
@@ -129,6 +133,129 @@ struct P32 {
 };
 
 inline size_t p32_pair_float4(int Vh) { return (size_t)((Vh + kTile - 1) / kTile) * 12 * kTile; }
+
+// FP16 pair-tiled field set with one float scale per site and right-hand side
+// (value = half * scale, |half| <= 1):
+//   uint4 P[pair][tile][component quarter q = k / 4][j % 32][k / 2 % 2]
+//   uint4 = components 2m, 2m + 1 as halves (re a, re b, im a, im b)
+//   float2 scale[pair][tile][j % 32] = (rhs a, rhs b)
+// A half2 is one operand pair of the FP32x2 instructions after one
+// conversion; a spinor pair is three 256-bit loads and one 64-bit load, half
+// the requests and 54 % of the bytes of the FP32 form.
+struct P16 {
+  using R = float;
+  static constexpr bool kScaled = true;
+  uint4 *p;
+  float2 *scale;
+  size_t pstride, sstride;  // uint4 and float2 per pair
+  __device__ __forceinline__ uint4 *at(int pr, int j) const {
+    return p + (size_t)pr * pstride + (size_t)(j >> 5) * (6 * kTile) + 2 * (j & (kTile - 1));
+  }
+  __device__ __forceinline__ float2 *scale_at(int pr, int j) const {
+    return scale + (size_t)pr * sstride + j;
+  }
+  __device__ __forceinline__ static void unpack(unsigned w, float2 &f) {
+    f = __half22float2(*reinterpret_cast<const __half2 *>(&w));
+  }
+  // the stored halves as floats, and the scales
+  __device__ __forceinline__ SpinorPair load_pair_raw(int pr, int j, float2 &nm) const {
+    const uint4 *q = at(pr, j);
+    nm = __ldg(scale_at(pr, j));
+    SpinorPair s;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      float4 a, b;
+      ldg_v8(reinterpret_cast<const float4 *>(q + m * 2 * kTile), a, b);
+      const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        CP &c = s.c[(4 * m + k) / 3][(4 * m + k) % 3];
+        unpack(__float_as_uint(w[2 * k]), c.re);
+        unpack(__float_as_uint(w[2 * k + 1]), c.im);
+      }
+    }
+    return s;
+  }
+  __device__ __forceinline__ SpinorPair load_pair(int pr, int j) const {
+    float2 nm;
+    SpinorPair s = load_pair_raw(pr, j, nm);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      CP &c = s.c[k / 3][k % 3];
+      c.re = __fmul2_rn(nm, c.re);
+      c.im = __fmul2_rn(nm, c.im);
+    }
+    return s;
+  }
+  // the scales of a spinor pair (its largest components) and their inverses
+  __device__ __forceinline__ static void scales(const SpinorPair &s, float2 &mx, float2 &inv) {
+    mx = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      const CP &c = s.c[k / 3][k % 3];
+      mx.x = fmaxf(mx.x, fmaxf(fabsf(c.re.x), fabsf(c.im.x)));
+      mx.y = fmaxf(mx.y, fmaxf(fabsf(c.re.y), fabsf(c.im.y)));
+    }
+    // below the smallest normal float a site is stored as zero: 1 / mx would overflow
+    if (!(mx.x >= 1.17549435e-38f)) mx.x = 0.f;
+    if (!(mx.y >= 1.17549435e-38f)) mx.y = 0.f;
+    inv = make_float2(mx.x > 0.f ? 1.f / mx.x : 0.f, mx.y > 0.f ? 1.f / mx.y : 0.f);
+  }
+  __device__ __forceinline__ static unsigned pack(float2 v, float2 inv) {
+    const float2 t = __fmul2_rn(v, inv);
+    const __half2 h = __floats2half2_rn(t.x, t.y);
+    return *reinterpret_cast<const unsigned *>(&h);
+  }
+  __device__ __forceinline__ void store_pair(int pr, int j, const SpinorPair &s) const {
+    float2 mx, inv;
+    scales(s, mx, inv);
+    uint4 *q = at(pr, j);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      float w[8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const CP &c = s.c[(4 * m + k) / 3][(4 * m + k) % 3];
+        w[2 * k] = __uint_as_float(pack(c.re, inv));
+        w[2 * k + 1] = __uint_as_float(pack(c.im, inv));
+      }
+      stg_v8(reinterpret_cast<float4 *>(q + m * 2 * kTile), make_float4(w[0], w[1], w[2], w[3]),
+             make_float4(w[4], w[5], w[6], w[7]));
+    }
+    *scale_at(pr, j) = mx;
+  }
+  __device__ __forceinline__ void store_lane(int pr, int lane, int j, const SpinorPair &s) const {
+    float2 mx, inv;
+    scales(s, mx, inv);
+    __half *q = reinterpret_cast<__half *>(at(pr, j)) + lane;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      const CP &c = s.c[k / 3][k % 3];
+      __half *d = q + (k / 4) * (2 * kTile * 8) + (k % 4) * 4;
+      d[0] = __float2half_rn(lane ? c.re.y * inv.y : c.re.x * inv.x);
+      d[2] = __float2half_rn(lane ? c.im.y * inv.y : c.im.x * inv.x);
+    }
+    reinterpret_cast<float *>(scale_at(pr, j))[lane] = lane ? mx.y : mx.x;
+  }
+  // per-rhs access (for the kernels that run once per reliable update)
+  __device__ __forceinline__ Spinor<float> load(int r, int j) const {
+    const SpinorPair f = load_pair(r >> 1, j);
+    const bool b = r & 1;
+    Spinor<float> s;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      const CP &c = f.c[k / 3][k % 3];
+      s.c[k / 3][k % 3] = cx(b ? c.re.y : c.re.x, b ? c.im.y : c.im.x);
+    }
+    return s;
+  }
+};
+
+// pair-tiled storage
+template <class SF>
+constexpr bool kPairTiled = std::is_same<SF, P32>::value || std::is_same<SF, P16>::value;
+
+inline size_t tile_count(int Vh) { return (size_t)((Vh + kTile - 1) / kTile); }
 
 // 18-real phased links, tiled: float2 U[idx / 32][mu][9][idx % 32]
 struct LT32f {
@@ -236,7 +363,8 @@ __device__ __forceinline__ double2 norm2_pair(const SpinorPair &v) {
   return n;
 }
 
-__device__ __forceinline__ void store_active(const P32 &f, int pr, int j, const SpinorPair &v,
+template <class PF>
+__device__ __forceinline__ void store_active(const PF &f, int pr, int j, const SpinorPair &v,
                                              bool act_a, bool act_b) {
   if (act_a && act_b)
     f.store_pair(pr, j, v);
@@ -244,23 +372,40 @@ __device__ __forceinline__ void store_active(const P32 &f, int pr, int j, const 
     f.store_lane(pr, act_a ? 0 : 1, j, v);
 }
 
-template <int MU, class LF>
-__device__ __forceinline__ void hop_pair_dir(SpinorPair &acc, const HopArgs<P32, LF> &A,
+// the scales of FP16 storage, on the projected half spinors (half the values)
+template <class PF>
+__device__ __forceinline__ void scale_half(HalfPair &h, float2 nm) {
+  if (PF::kScaled) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        h.c[b][c].re = __fmul2_rn(nm, h.c[b][c].re);
+        h.c[b][c].im = __fmul2_rn(nm, h.c[b][c].im);
+      }
+  }
+}
+
+template <int MU, class PF, class LF>
+__device__ __forceinline__ void hop_pair_dir(SpinorPair &acc, const HopArgs<PF, LF> &A,
                                              const SiteCoord &cd, int pr, int self, int qoff,
                                              bool g5in) {
   const Geom &g = A.eg.g;
+  float2 nm;
   {  // backward: (1 + g_mu) U_mu(x-mu)^+ in(x-mu)
     const int j = nb_lex(g, cd, MU, -1) >> 1;
     const Link<float> W = A.links.load(MU, qoff + j);
-    const SpinorPair f = A.in.load_pair(pr, j);
-    const HalfPair h = g5in ? project_pair<MU, -1>(f) : project_pair<MU, +1>(f);
+    const SpinorPair f = A.in.load_pair_raw(pr, j, nm);
+    HalfPair h = g5in ? project_pair<MU, -1>(f) : project_pair<MU, +1>(f);
+    scale_half<PF>(h, nm);
     accum_recon_pair(MU, +1, acc, link_mul_pair<true>(W, h));
   }
   {  // forward: (1 - g_mu) U_mu(x) in(x+mu)
     const int j = nb_lex(g, cd, MU, +1) >> 1;
     const Link<float> W = A.links.load(MU, self);
-    const SpinorPair f = A.in.load_pair(pr, j);
-    const HalfPair h = g5in ? project_pair<MU, +1>(f) : project_pair<MU, -1>(f);
+    const SpinorPair f = A.in.load_pair_raw(pr, j, nm);
+    HalfPair h = g5in ? project_pair<MU, +1>(f) : project_pair<MU, -1>(f);
+    scale_half<PF>(h, nm);
     accum_recon_pair(MU, -1, acc, link_mul_pair<false>(W, h));
   }
 }
@@ -273,8 +418,8 @@ __device__ __forceinline__ void hop_pair_dir(SpinorPair &acc, const HopArgs<P32,
 // RUPD: the sweep that produces A p of a CG iteration updates the residual
 // instead, r -= alpha A p, and its partials are those of |r|^2; A p itself
 // is not stored (CG needs it for nothing else).
-template <class LF, bool G5IN, bool G5HOP, bool AUX, bool RUPD = false>
-__global__ void __launch_bounds__(kHopMaxThreads, 2) k_eo_hop_pt(HopArgs<P32, LF> A) {
+template <class PF, class LF, bool G5IN, bool G5HOP, bool AUX, bool RUPD = false>
+__global__ void __launch_bounds__(kHopMaxThreads, 2) k_eo_hop_pt(HopArgs<PF, LF> A) {
   const int pr = blockIdx.x * blockDim.y + threadIdx.y;
   const int ra = 2 * pr;
   if (ra >= A.nrhs) return;

@@ -42,7 +42,7 @@ namespace {
 // Right-hand sides per batch: up to 96, so that the 8 x 12 columns of the
 // benchmark can advance as one set (each link loaded once per site for all).
 constexpr int kMaxBatch = 96;
-// Tuner keys of the pair-tiled FP32 fields: precision + kPairKey.
+// Tuner keys of the pair-tiled fields: precision + kPairKey.
 constexpr int kPairKey = 10;
 constexpr size_t kMaxStagedSmem = 200 * 1024;  // opt-in dynamic shared memory of the staged stencil
 
@@ -241,6 +241,33 @@ __global__ void __launch_bounds__(kUpdTiles * 192)
   stg_v8(p.at(pr, s) + off, q[0], q[1]);
 }
 
+// the same with FP16 p and r (thread = site x rhs pair: a site's scale needs
+// all its components)
+__global__ void k_p_upd_pt(P16 p, P16 rs, P32 xs, Scal S, int nsites, int nrhs) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x, pr = blockIdx.y;
+  const int ra = 2 * pr;
+  if (s >= nsites) return;
+  const bool act_a = !S.done[ra];
+  const bool act_b = ra + 1 < nrhs && !S.done[ra + 1];
+  if (!act_a && !act_b) return;
+  const float2 a = make_float2((float)S.alpha[ra], act_b ? (float)S.alpha[ra + 1] : 0.f);
+  const float2 b = make_float2((float)S.beta[ra], act_b ? (float)S.beta[ra + 1] : 0.f);
+  const SpinorPair rv = rs.load_pair(pr, s);
+  SpinorPair pv = p.load_pair(pr, s);
+  SpinorPair xv = xs.load_pair(pr, s);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      xv.c[k][c].re = __ffma2_rn(a, pv.c[k][c].re, xv.c[k][c].re);
+      xv.c[k][c].im = __ffma2_rn(a, pv.c[k][c].im, xv.c[k][c].im);
+      pv.c[k][c].re = __ffma2_rn(b, pv.c[k][c].re, rv.c[k][c].re);
+      pv.c[k][c].im = __ffma2_rn(b, pv.c[k][c].im, rv.c[k][c].im);
+    }
+  store_active(xs, pr, s, xv, act_a, act_b);
+  store_active(p, pr, s, pv, act_a, act_b);
+}
+
 // Pair-tiled forms of the reliable-update kernels below: thread = site x rhs
 // pair, so each pair-tiled field is read once (the per-rhs forms read both
 // lanes of every float4 for one rhs).  skip[r] != 0 leaves rhs r unchanged.
@@ -291,7 +318,8 @@ __global__ void k_absorb_pt(F64Acc x64, P32 xs, const double *scale, const int *
 }
 
 // sloppy <- scale * FP64
-__global__ void k_to_sloppy_pt(P32 dst, F64Acc src, const double *scale, const int *skip,
+template <class PF>
+__global__ void k_to_sloppy_pt(PF dst, F64Acc src, const double *scale, const int *skip,
                                int nsites, int nrhs) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int pr = blockIdx.y;
@@ -326,7 +354,8 @@ __global__ void k_to_sloppy_pt(P32 dst, F64Acc src, const double *scale, const i
 }
 
 // p = p - r_s (the kept direction q, see k_dir_strip)
-__global__ void k_dir_strip_pt(P32 p, P32 rs, const int *skip, int nsites, int nrhs) {
+template <class PF>
+__global__ void k_dir_strip_pt(PF p, PF rs, const int *skip, int nsites, int nrhs) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int pr = blockIdx.y;
   const PairLanes m = pair_lanes(pr, nrhs, skip);
@@ -344,7 +373,8 @@ __global__ void k_dir_strip_pt(P32 p, P32 rs, const int *skip, int nsites, int n
 }
 
 // p = (a - i b) r_s' + u q, per-lane coefficients as in k_dir_restore
-__global__ void k_dir_restore_pt(P32 p, P32 rs, Scal S, const int *skip, int nsites, int nrhs) {
+template <class PF>
+__global__ void k_dir_restore_pt(PF p, PF rs, Scal S, const int *skip, int nsites, int nrhs) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int pr = blockIdx.y;
   const PairLanes m = pair_lanes(pr, nrhs, skip);
@@ -382,7 +412,8 @@ __global__ void k_dir_restore_pt(P32 p, P32 rs, Scal S, const int *skip, int nsi
   store_active(p, pr, s, pv, m.act_a, m.act_b);
 }
 
-__global__ void k_copy_pt(P32 dst, P32 src, const int *skip, int nsites, int nrhs) {
+template <class PF>
+__global__ void k_copy_pt(PF dst, PF src, const int *skip, int nsites, int nrhs) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int pr = blockIdx.y;
   const PairLanes m = pair_lanes(pr, nrhs, skip);
@@ -393,8 +424,9 @@ __global__ void k_copy_pt(P32 dst, P32 src, const int *skip, int nsites, int nrh
 // <a, b> = sum conj(a) b per rhs, real and imaginary parts from one pass:
 // blockIdx.y = pair; partials[(2 rhs + part) * kMaxRedBlocks + block]
 // (part 0 real, 1 imaginary); the last block writes re[r], im[r].
+template <class PF>
 __global__ void __launch_bounds__(kRedThreads)
-    k_cdot_pt(P32 a, P32 b, int nsites, int nrhs, double *partials, unsigned *counters,
+    k_cdot_pt(PF a, PF b, int nsites, int nrhs, double *partials, unsigned *counters,
               const int *__restrict__ skip, double *re, double *im) {
   const int pr = blockIdx.y;
   const PairLanes m = pair_lanes(pr, nrhs, skip);
@@ -713,6 +745,7 @@ template <> constexpr double spinor_bytes<F64Acc>() { return 192; }
 template <> constexpr double spinor_bytes<F32Acc>() { return 96; }
 template <> constexpr double spinor_bytes<F16Acc>() { return 52; }  // 48 + float norm
 template <> constexpr double spinor_bytes<P32>() { return 96; }
+template <> constexpr double spinor_bytes<P16>() { return 52; }
 
 int red_blocks_sites(int n) {
   int b = (n + kRedThreads * 2 - 1) / (kRedThreads * 2);
@@ -791,7 +824,7 @@ struct Batch {
       CVCB_CUDA(cudaEventRecordWithFlags(rec.a, L->stream, capturing ? cudaEventRecordExternal : 0));
     }
     bool packed = false;
-    if constexpr (std::is_same<AF, P32>::value) {  // pair-tiled fields
+    if constexpr (kPairTiled<AF>) {  // pair-tiled fields
       CVCB_TRY((launch_pt<LL, G5IN, G5HOP, AUX, false>(a, sh)));
       packed = true;
     } else if constexpr (sizeof(typename AF::R) == 4) {
@@ -800,7 +833,7 @@ struct Batch {
         packed = true;
       }
     }
-    if constexpr (std::is_same<AF, P32>::value) {
+    if constexpr (kPairTiled<AF>) {
     } else if (packed) {
     } else if (by > 1 && sh.nr == 1) {
       // rows of the block share links staged in shared memory
@@ -833,7 +866,7 @@ struct Batch {
         default: k_eo_hop<AF, LL, 1, G5IN, G5HOP, AUX><<<grid, block, 0, L->stream>>>(a); break;
       }
     }
-    if (!std::is_same<AF, P32>::value) CVCB_LAUNCHED(L);  // launch_pt counts its own
+    if (!kPairTiled<AF>) CVCB_LAUNCHED(L);  // launch_pt counts its own
     if (rec_this) {
       CVCB_CUDA(cudaEventRecordWithFlags(rec.b, L->stream, capturing ? cudaEventRecordExternal : 0));
       rec.bytes_per_rhs = (double)g.Vh * spinor_bytes<AF>() * (AUX ? 3 : 2);
@@ -847,7 +880,7 @@ struct Batch {
   // update of CG: r_s -= alpha (A(-mu) yo + 1/2 g5 H_oe te2) and per-warp
   // partials of |r_s|^2 (A p itself is not stored)
   int hop_rupd(SF in, SF aux, double d2a, double d2b) {
-    if constexpr (std::is_same<SF, P32>::value) {
+    if constexpr (kPairTiled<SF>) {
       HopArgs<SF, LF> a{rs, in, aux, links, EoGeom{g, 1}, n, S.done, 1, 0, d2a, d2b, 0.5};
       if (!dot_fusable()) {
         set_error("fused residual update needs warp-aligned blocks");
@@ -908,19 +941,21 @@ struct Batch {
   }
 
   // Pair-tiled stencil launch
-  template <class LL, bool G5IN, bool G5HOP, bool AUX, bool RUPD>
-  int launch_pt(const HopArgs<P32, LL> &a, const LaunchShape &sh) {
+  template <class LL, bool G5IN, bool G5HOP, bool AUX, bool RUPD, class PF>
+  int launch_pt(const HopArgs<PF, LL> &a, const LaunchShape &sh) {
     const int groups = (n + 1) / 2;
-    if (sh.pk == 2) {
-      dim3 grid(groups, std::min((g.Vh + kTile - 1) / kTile, 65535));
-      k_eo_hop_sp<LL, G5IN, G5HOP, AUX, RUPD><<<grid, kSplitThreads, 0, L->stream>>>(a);
-      CVCB_LAUNCHED(L);
-      return CVCB_OK;
+    if constexpr (std::is_same<PF, P32>::value) {
+      if (sh.pk == 2) {
+        dim3 grid(groups, std::min((g.Vh + kTile - 1) / kTile, 65535));
+        k_eo_hop_sp<LL, G5IN, G5HOP, AUX, RUPD><<<grid, kSplitThreads, 0, L->stream>>>(a);
+        CVCB_LAUNCHED(L);
+        return CVCB_OK;
+      }
     }
     const int by = std::min(sh.by, groups);
     const int site_blocks = (g.Vh + sh.bx - 1) / sh.bx;
     dim3 block(sh.bx, by), grid((groups + by - 1) / by, std::min(site_blocks, 65535));
-    k_eo_hop_pt<LL, G5IN, G5HOP, AUX, RUPD><<<grid, block, 0, L->stream>>>(a);
+    k_eo_hop_pt<PF, LL, G5IN, G5HOP, AUX, RUPD><<<grid, block, 0, L->stream>>>(a);
     CVCB_LAUNCHED(L);
     return CVCB_OK;
   }
@@ -945,7 +980,7 @@ struct Batch {
 
   // one CG iteration (sloppy)
   int iteration() {
-    if constexpr (std::is_same<SF, P32>::value) {
+    if constexpr (kPairTiled<SF>) {
       // pair-tiled fields: alpha = |r|^2 / |M p|^2 between the two
       // applications of M, and the last sweep updates r itself
       const int np = (n + 1) / 2;
@@ -965,28 +1000,33 @@ struct Batch {
         k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, dot_np, EpiBetaB{S}, S.done);
         CVCB_LAUNCHED(L);
       }
-      const int ub = ((g.Vh + kTile - 1) / kTile + kUpdTiles - 1) / kUpdTiles;
-      k_p_upd_pt<<<dim3(ub, np), kUpdTiles * 192, 0, L->stream>>>(p, rs, xs, S, g.Vh, n);
+      const int tiles = (g.Vh + kTile - 1) / kTile;
+      if constexpr (std::is_same<SF, P32>::value)
+        k_p_upd_pt<<<dim3((tiles + kUpdTiles - 1) / kUpdTiles, np), kUpdTiles * 192, 0, L->stream>>>(
+            p, rs, xs, S, g.Vh, n);
+      else
+        k_p_upd_pt<<<dim3((tiles + 3) / 4, np), 4 * kTile, 0, L->stream>>>(p, rs, xs, S, g.Vh, n);
+      CVCB_LAUNCHED(L);
+      return CVCB_OK;
+    } else {
+      dim3 rg(red_blocks_sites(g.Vh), n);
+      if (dot_fusable()) {
+        CVCB_TRY(normal_op_sloppy(Ap, p, S.done, dot_part));
+        k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, dot_np, EpiAlphaB{S}, S.done);
+      } else {
+        CVCB_TRY(normal_op_sloppy(Ap, p, S.done));
+        k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedPAp<SF>{p, Ap}, EpiAlphaB{S}, g.Vh, br,
+                                                        S.done);
+      }
+      CVCB_LAUNCHED(L);
+      k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedUpdate<SF>{Ap, rs, S},
+                                                      EpiBetaB{S}, g.Vh, br, S.done);
+      CVCB_LAUNCHED(L);
+      dim3 eg((g.Vh + 127) / 128, n);
+      k_p_upd<<<eg, 128, 0, L->stream>>>(p, rs, xs, S, g.Vh, n);
       CVCB_LAUNCHED(L);
       return CVCB_OK;
     }
-    dim3 rg(red_blocks_sites(g.Vh), n);
-    if (dot_fusable()) {
-      CVCB_TRY(normal_op_sloppy(Ap, p, S.done, dot_part));
-      k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, dot_np, EpiAlphaB{S}, S.done);
-    } else {
-      CVCB_TRY(normal_op_sloppy(Ap, p, S.done));
-      k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedPAp<SF>{p, Ap}, EpiAlphaB{S}, g.Vh, br,
-                                                      S.done);
-    }
-    CVCB_LAUNCHED(L);
-    k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedUpdate<SF>{Ap, rs, S},
-                                                    EpiBetaB{S}, g.Vh, br, S.done);
-    CVCB_LAUNCHED(L);
-    dim3 eg((g.Vh + 127) / 128, n);
-    k_p_upd<<<eg, 128, 0, L->stream>>>(p, rs, xs, S, g.Vh, n);
-    CVCB_LAUNCHED(L);
-    return CVCB_OK;
   }
 
   // FP64: out_o = M(m) in_o  (t64 even half as intermediate)
@@ -1028,7 +1068,7 @@ struct Batch {
     k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedRhat{f64(bh64, 1), f64(y64, 1)},
                                                     EpiRhat{S}, g.Vh, br, ru_skip);
     CVCB_LAUNCHED(L);
-    if constexpr (std::is_same<SF, P32>::value)
+    if constexpr (kPairTiled<SF>)
       k_to_sloppy_pt<<<dim3(eg.x, (n + 1) / 2), 128, 0, L->stream>>>(yo, f64(y64, 1), S.scale,
                                                                       ru_skip, g.Vh, n);
     else
@@ -1060,6 +1100,11 @@ template <>
 P32 make_sloppy<P32>(void *base, size_t Vh, int, float *) {
   return P32{static_cast<float4 *>(base), p32_pair_float4((int)Vh)};
 }
+template <>
+P16 make_sloppy<P16>(void *base, size_t Vh, int, float *norm) {
+  const size_t tiles = tile_count((int)Vh);
+  return P16{static_cast<uint4 *>(base), reinterpret_cast<float2 *>(norm), tiles * 6 * kTile, tiles * kTile};
+}
 
 template <class SF>
 size_t sloppy_site_bytes();
@@ -1069,15 +1114,19 @@ template <>
 size_t sloppy_site_bytes<F16Acc>() { return 48; }
 template <>
 size_t sloppy_site_bytes<F64Acc>() { return 192; }
-template <>
-size_t sloppy_site_bytes<P32>() { return 96; }
-
 // Bytes of one sloppy field set of n right-hand sides (pair-tiled sets hold
-// whole pairs of whole tiles).
+// whole pairs of whole tiles), and of its per-site scales.
 template <class SF>
 size_t sloppy_field_bytes(size_t Vh, int n) {
-  if (std::is_same<SF, P32>::value) return p32_pair_float4((int)Vh) * sizeof(float4) * ((n + 1) / 2);
-  return sloppy_site_bytes<SF>() * Vh * n;
+  if constexpr (kPairTiled<SF>)
+    return tile_count((int)Vh) * kTile * (std::is_same<SF, P16>::value ? 96 : 192) * ((n + 1) / 2);
+  else
+    return sloppy_site_bytes<SF>() * Vh * n;
+}
+template <class SF>
+size_t sloppy_scale_bytes(size_t Vh, int n) {
+  if (std::is_same<SF, P16>::value) return tile_count((int)Vh) * kTile * sizeof(float2) * ((n + 1) / 2);
+  return std::is_same<SF, F16Acc>::value ? sizeof(float) * Vh * n : 0;
 }
 
 template <class LF>
@@ -1144,13 +1193,13 @@ int setup_batch(cvcb_lattice *L, Batch<SF, XF, LF> &B, int n, bool with_fp64 = t
   const size_t f64 = with_fp64 ? (size_t)12 * g.V * sizeof(double2) * n : 0;
   const size_t sl = sloppy_field_bytes<SF>(g.Vh, n);
   const size_t xsl = sloppy_field_bytes<XF>(g.Vh, n);
-  const size_t nrm = sizeof(float) * (size_t)g.Vh * n;
+  const size_t nrm = sloppy_scale_bytes<SF>(g.Vh, n);
   auto rnd = [](size_t b) { return (b + 255) & ~size_t(255); };  // every piece 256-aligned
   const size_t scal = 8 * rnd(sizeof(double) * kMaxBatch) + 3 * rnd(sizeof(int) * kMaxBatch);
   const size_t part = rnd(sizeof(double) * kMaxRedBlocks * kMaxBatch * 2) +
                       rnd(sizeof(unsigned) * kMaxBatch);
   const size_t dotb = sizeof(double) * (size_t)n * (g.Vh / 32 + 64);
-  const size_t total = 5 * rnd(f64) + 6 * (rnd(sl) + rnd(nrm)) + rnd(xsl) + rnd(nrm) + scal + part +
+  const size_t total = 5 * rnd(f64) + 6 * (rnd(sl) + rnd(nrm)) + rnd(xsl) + scal + part +
                        rnd(dotb);
   void *mem;
   CVCB_TRY(ensure_buffer(L, SLOT_MIX0, total, &mem));
@@ -1173,8 +1222,7 @@ int setup_batch(cvcb_lattice *L, Batch<SF, XF, LF> &B, int n, bool with_fp64 = t
   }
   {
     void *b = take(xsl);
-    float *nb = (float *)take(nrm);
-    B.xs = make_sloppy<XF>(b, g.Vh, n, nb);
+    B.xs = make_sloppy<XF>(b, g.Vh, n, nullptr);
     B.xs_mem = b;
     B.xs_bytes = xsl;
   }
@@ -1229,11 +1277,11 @@ int time_ms(cvcb_lattice *L, Fn fn, int reps, float *best) {
 template <class SF, class XF, class LF>
 int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int block_threads = 0) {
   if (block_threads > 0) {  // caller's choice: that many sites per block, one rhs (pair) per thread
-    B.shape = std::is_same<SF, P32>::value ? LaunchShape{block_threads, 1, 2, 1}
+    B.shape = kPairTiled<SF> ? LaunchShape{block_threads, 1, 2, 1}
                                            : LaunchShape{block_threads, 1, 1};
     return CVCB_OK;
   }
-  constexpr bool pairs = std::is_same<SF, P32>::value;
+  constexpr bool pairs = kPairTiled<SF>;
   auto key = std::make_tuple(L->g.V, prec + (pairs ? kPairKey : 0), recon, B.n);
   auto it = g_tuned_shape.find(key);
   if (it != g_tuned_shape.end()) {
@@ -1251,7 +1299,7 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
       if (sizeof(typename SF::R) == 8) f.nr = 1, f.pk = 0;
       if (pairs) {  // one rhs pair per thread; 4th field 2: directions on warps
         f.nr = 2;
-        f.pk = nf >= 4 && f.pk == 2 ? 2 : 1;
+        f.pk = nf >= 4 && f.pk == 2 && std::is_same<SF, P32>::value ? 2 : 1;
         if (f.pk == 2) f.bx = kTile, f.by = 1;
       }
       B.shape = f;
@@ -1291,7 +1339,7 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
         best = B.shape;
       }
     }
-  if (pairs) {  // a site's directions on eight warps
+  if (std::is_same<SF, P32>::value) {  // a site's directions on eight warps
     B.shape = LaunchShape{kTile, 1, 2, 2};
     float ms;
     if (time_ms(L, [&] { return B.normal_op_sloppy(B.Ap, B.p, nullptr); }, 3, &ms) != CVCB_OK)
@@ -1373,7 +1421,7 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
   CVCB_TRY(B.reliable_update(false));
   // x_s = 0 (all-zero bits are 0.0), p = r_s
   CVCB_CUDA(cudaMemsetAsync(B.xs_mem, 0, B.xs_bytes, L->stream));
-  if constexpr (std::is_same<SF, P32>::value)
+  if constexpr (kPairTiled<SF>)
     k_copy_pt<<<dim3(eg.x, (n + 1) / 2), 128, 0, L->stream>>>(B.p, B.rs, nullptr, g.Vh, n);
   else
     k_copy<<<eg, 128, 0, L->stream>>>(B.p, B.rs, nullptr, g.Vh, n);
@@ -1463,7 +1511,7 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
   // delta 0: by the storage of the inner iterations -- an FP16 recursion
   // drifts from the true residual after about three decades, FP32 after six
   const double delta = P->delta > 0 ? P->delta
-                       : std::is_same<SF, F16Acc>::value ? 0.1
+                       : std::is_same<SF, F16Acc>::value || std::is_same<SF, P16>::value ? 0.1
                        : sizeof(typename SF::R) == 4 ? 1e-4 : 1e-8;
   const double delta2 = delta * delta;
   int total_iter = 0, nru = 0, nrestart = 0;
@@ -1530,13 +1578,13 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
     // keep the search direction: q = p - r_s now, p = r_s' + q (q orthogonalised
     // against r_s') after the update
     const dim3 egp(eg.x, (n + 1) / 2);  // pair-tiled fields: one thread per site and pair
-    if constexpr (std::is_same<SF, P32>::value)
+    if constexpr (kPairTiled<SF>)
       k_dir_strip_pt<<<egp, 128, 0, L->stream>>>(B.p, B.rs, B.ru_skip, g.Vh, n);
     else
       k_dir_strip<<<eg, 128, 0, L->stream>>>(B.p, B.rs, B.ru_skip, g.Vh, n);
     CVCB_LAUNCHED(L);
     CVCB_TRY(B.reliable_update(true));
-    if constexpr (std::is_same<SF, P32>::value) {
+    if constexpr (kPairTiled<SF>) {
       k_cdot_pt<<<dim3(rg.x, (n + 1) / 2), kRedThreads, 0, L->stream>>>(
           B.rs, B.p, g.Vh, n, B.br.partials, B.br.counters, B.ru_skip, B.S.pAp, B.S.alpha);
       CVCB_LAUNCHED(L);
@@ -1559,7 +1607,7 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
     }
     if (restart) {
       CVCB_TRY(put_flags(L, B.rst_skip, rst, n));
-      if constexpr (std::is_same<SF, P32>::value)
+      if constexpr (kPairTiled<SF>)
         k_copy_pt<<<egp, 128, 0, L->stream>>>(B.p, B.rs, B.rst_skip, g.Vh, n);
       else
         k_copy<<<eg, 128, 0, L->stream>>>(B.p, B.rs, B.rst_skip, g.Vh, n);
@@ -1709,9 +1757,14 @@ int sloppy_normal_op(cvcb_lattice *L, int prec, int recon, int layout, int n,
                      : sloppy_normal_op_t<F16Acc, F32Acc, L32f>(L, prec, recon, n, in, out);
 }
 
-// FP32 inner iterations on pair-tiled fields (k_eo_hop_pt and the pair CG
-// kernels), the default; CVCB_PAIRS=0 selects the per-rhs fields with the
-// packed-pair stencil k_eo_hop_x2 instead (read once per process).
+// Inner iterations on pair-tiled fields (k_eo_hop_pt and the pair CG kernels),
+// the default for FP32 and FP16 storage; CVCB_PAIRS=0 selects the per-rhs
+// fields with the packed-pair stencil k_eo_hop_x2 instead (read once per
+// process).  FP16: 12 columns at 16^3x32 take 21.5 ms against 23.7 with the
+// per-rhs fields (M^+M 220 against 247 us), whose links are FP16 too; the pair
+// kernels read the FP32 ones, shared by the pair.  A sweep takes as long as
+// in FP32 with half the requests and bytes: latency at 16 warps per SM and
+// the FMA pipe (50 % busy) bound it, not its traffic.
 bool use_pairs() {
   static const bool on = [] {
     const char *e = getenv("CVCB_PAIRS");
@@ -1756,6 +1809,9 @@ int time_stencil(cvcb_lattice *L, int kind, int prec, int recon, int nrhs, int r
   if (prec == CVCB_PREC_SINGLE && use_pairs())
     return recon == 12 ? time_stencil_t<P32, P32, LT32c>(L, kind, prec, recon, nrhs, reps, ms)
                        : time_stencil_t<P32, P32, LT32f>(L, kind, prec, recon, nrhs, reps, ms);
+  if (use_pairs())
+    return recon == 12 ? time_stencil_t<P16, P32, LT32c>(L, kind, prec, recon, nrhs, reps, ms)
+                       : time_stencil_t<P16, P32, LT32f>(L, kind, prec, recon, nrhs, reps, ms);
   if (prec == CVCB_PREC_SINGLE)
     return recon == 12 ? time_stencil_t<F32Acc, F32Acc, L32c>(L, kind, prec, recon, nrhs, reps, ms)
                        : time_stencil_t<F32Acc, F32Acc, L32f>(L, kind, prec, recon, nrhs, reps, ms);
@@ -1903,7 +1959,7 @@ int solve_batched(cvcb_lattice *L, double *const *x, const double *const *b, int
     host_fields = !is_device_ptr(x[i]) && !is_device_ptr(b[i]);
   int nb = P->block_rhs;
   if (!nb) {
-    const bool pairs = P->precision == CVCB_PREC_SINGLE && use_pairs();
+    const bool pairs = P->precision != CVCB_PREC_DOUBLE && use_pairs();
     auto key = std::make_tuple(L->g.V,
                                P->precision + (pairs ? kPairKey : 0) + (host_fields ? 100 : 0),
                                recon, nrhs);
@@ -1915,9 +1971,12 @@ int solve_batched(cvcb_lattice *L, double *const *x, const double *const *b, int
       const bool hf = host_fields;
       if (P->precision == CVCB_PREC_DOUBLE)
         rc = tune_batch<F64Acc, F64Acc, L64>(L, P, recon, nrhs, hf, &nb);
-      else if (pairs)
+      else if (pairs && P->precision == CVCB_PREC_SINGLE)
         rc = recon == 12 ? tune_batch<P32, P32, LT32c>(L, P, recon, nrhs, hf, &nb)
                          : tune_batch<P32, P32, LT32f>(L, P, recon, nrhs, hf, &nb);
+      else if (pairs)
+        rc = recon == 12 ? tune_batch<P16, P32, LT32c>(L, P, recon, nrhs, hf, &nb)
+                         : tune_batch<P16, P32, LT32f>(L, P, recon, nrhs, hf, &nb);
       else if (P->precision == CVCB_PREC_SINGLE)
         rc = recon == 12 ? tune_batch<F32Acc, F32Acc, L32c>(L, P, recon, nrhs, hf, &nb)
                          : tune_batch<F32Acc, F32Acc, L32f>(L, P, recon, nrhs, hf, &nb);
@@ -1935,6 +1994,9 @@ int solve_batched(cvcb_lattice *L, double *const *x, const double *const *b, int
     if (P->precision == CVCB_PREC_SINGLE && use_pairs())
       return recon == 12 ? run_batch<P32, P32, LT32c>(L, xs, bs, n, P, st, nullptr, read)
                          : run_batch<P32, P32, LT32f>(L, xs, bs, n, P, st, nullptr, read);
+    if (use_pairs())
+      return recon == 12 ? run_batch<P16, P32, LT32c>(L, xs, bs, n, P, st, nullptr, read)
+                         : run_batch<P16, P32, LT32f>(L, xs, bs, n, P, st, nullptr, read);
     if (P->precision == CVCB_PREC_SINGLE)
       return recon == 12 ? run_batch<F32Acc, F32Acc, L32c>(L, xs, bs, n, P, st, nullptr, read)
                          : run_batch<F32Acc, F32Acc, L32f>(L, xs, bs, n, P, st, nullptr, read);
@@ -1994,7 +2056,7 @@ int cvcb_tuned_shape(cvcb_lattice *L, int precision, int link_recon, int nrhs, i
                      int *rows_per_block, int *rhs_per_thread, int *variant) {
   if (!L || !sites_per_block || !rows_per_block || !rhs_per_thread || !variant)
     return CVCB_ERR_NULL;
-  const bool pairs = precision == CVCB_PREC_SINGLE && cvcb::use_pairs();
+  const bool pairs = precision != CVCB_PREC_DOUBLE && cvcb::use_pairs();
   auto it = cvcb::g_tuned_shape.find(std::make_tuple(
       L->g.V, precision + (pairs ? cvcb::kPairKey : 0), link_recon, nrhs));
   if (it == cvcb::g_tuned_shape.end()) {

@@ -73,6 +73,19 @@ def test_stencil_variants_agree(prec):
         assert abs(r["x4"] - base["x4"]) <= 1e-8 * base["x4"], (v, r, base)
 
 
+@pytest.mark.parametrize("recon", [12, 18])
+def test_half_pairs_agree(recon):
+    """FP16 fields tiled by rhs pairs (11 rhs: a lone last one) against the
+    per-rhs FP16 fields: the same solutions, and no more iterations than the
+    tolerance of the other variants (the links are FP32 instead of FP16)."""
+    base = run(2, "64,1,2,1", 0, recon)
+    for shape in ("64,1,2,1", "32,2,2,1"):
+        r = run(2, shape, 1, recon)
+        assert r["conv"] == 11 and r["res"] <= 1e-10 and r["chk"] <= 1e-10, r
+        assert r["iters"] <= 1.1 * base["iters"], (r, base)
+        assert abs(r["x4"] - base["x4"]) <= 1e-8 * base["x4"], (r, base)
+
+
 SPLIT_CHILD = r"""
 import sys
 import numpy as np
