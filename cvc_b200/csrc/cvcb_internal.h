@@ -161,7 +161,8 @@ struct SolverScalars {
   int done;       // 1: converged, 2: breakdown (non-finite scalar)
   int niter;      // iteration at which done was set
   int iter;       // iterations started
-  int pad;
+  int itmax;      // the caller's limit
+  int xlast;      // iteration whose solution step stands although done is set
 };
 
 // ---- the context -----------------------------------------------------------
@@ -257,8 +258,11 @@ enum BufSlot {
 // dslash.cu: full-lattice FP64 twisted-mass operator, device layout.
 //   out = a*in + i*b*g5*in + c*H in   (then g5 applied to out if g5out)
 // H in = sum_mu [(1-g_mu) U_mu(x) in(x+mu) + (1+g_mu) U_mu(x-mu)^+ in(x-mu)]
+// `dot`: scalar products taken along (bicgstab.cuh), may be null.
+struct TmDot;
 int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, double b, double c,
-                   bool g5out, const int *done_flag);
+                   bool g5out, const int *done_flag, const TmDot *dot = nullptr);
+int tm_full_blocks(const Geom &g);  // partial sums of a TmDot: 3 per block
 // the same on CVC-layout device arrays (16-byte aligned, not overlapping)
 int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a, double b, double c,
                        bool g5out);

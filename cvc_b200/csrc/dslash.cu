@@ -13,17 +13,67 @@
 // HBM-bound: per site it must read 8 neighbour spinors (mostly L1/L2 hits:
 // each spinor is used by 8 sites), 8 links (each used by 2 sites), its own
 // spinor, and write one spinor.  Compulsory traffic 2*192 + 4*144 = 960 B.
+#include "bicgstab.cuh"
 #include "cvcb_internal.h"
 #include "spinor_ops.cuh"
 
 namespace cvcb {
 
-template <bool G5OUT, int NT, int MINB>
+// DOT: the scalar products that BiCGStab takes of the result (TmDot) come from
+// the registers of the sweep: one field read instead of two and a launch
+// less.  Per-block partials, summed by the last block in block order.
+template <int NT>
+__device__ __forceinline__ void tm_dot_finish(const TmDot &D, double (&v)[3]) {
+  __shared__ double sh[3][NT / 32];
+  __shared__ bool last;
+  auto reduce = [&] {
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) sh[q][threadIdx.x >> 5] = v[q];
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        v[q] = sh[q][0];
+        for (int w = 1; w < NT / 32; ++w) v[q] += sh[q][w];
+      }
+  };
+  reduce();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) D.partials[(size_t)blockIdx.x * 3 + q] = v[q];
+    __threadfence();
+    last = atomicAdd(D.counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int q = 0; q < 3; ++q) v[q] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += NT)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) v[q] += __ldcg(D.partials + (size_t)b * 3 + q);
+  __syncthreads();
+  reduce();
+  if (threadIdx.x == 0) {
+    *D.counter = 0;
+    if (D.kind == 1)
+      epi_alpha(D.S, v[0], v[1]);
+    else
+      epi_omega(D.S, v[0], v[1], v[2]);
+  }
+}
+
+template <bool G5OUT, bool DOT, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_tm_full_f64(double2 *__restrict__ out,
                                                      const double2 *__restrict__ in,
                                                      const double2 *__restrict__ U, Geom g,
                                                      double a, double b, double c,
-                                                     const int *__restrict__ done) {
+                                                     const int *__restrict__ done, TmDot D) {
   if (done && *done) return;
   // Blocks alternate between the parities (block 2k: even sites of range k,
   // block 2k+1: odd sites of range k).  A link serves the forward hop of one
@@ -32,7 +82,8 @@ __global__ void __launch_bounds__(NT, MINB) k_tm_full_f64(double2 *__restrict__ 
   // L2, where parity after parity would read all links from DRAM twice.
   const int p = blockIdx.x & 1;
   const int i = (blockIdx.x >> 1) * blockDim.x + threadIdx.x;
-  if (i >= g.Vh) return;
+  double dv[3] = {0.0, 0.0, 0.0};
+  if (i < g.Vh) {
   const int s = p * g.Vh + i;
   const SiteCoord cd = site_coord(g, p, i);
   const size_t V = g.V;
@@ -76,39 +127,53 @@ __global__ void __launch_bounds__(NT, MINB) k_tm_full_f64(double2 *__restrict__ 
     }
   }
   store_spinor(out, V, s, r);
+  if (DOT) {
+    const Spinor<double> f2 = load_spinor(D.f, V, s);
+    Cx<double> d = cx(0.0, 0.0);
+#pragma unroll
+    for (int sp = 0; sp < 4; ++sp)
+#pragma unroll
+      for (int co = 0; co < 3; ++co) {
+        const Cx<double> o = r.c[sp][co];
+        cfmac(d, f2.c[sp][co], o);  // <f, out>
+        dv[2] = fma(o.re, o.re, dv[2]);
+        dv[2] = fma(o.im, o.im, dv[2]);
+      }
+    dv[0] = d.re;
+    dv[1] = D.kind == 1 ? d.im : -d.im;  // kind 2: <out, f>
+  }
+  }  // i < Vh
+  if (DOT) tm_dot_finish<NT>(D, dv);
 }
 
-// Launch variants (threads per block, minimum resident blocks per SM); the
-// second number caps the registers per thread.  The variant is chosen once
-// per process by timing (tm_full_variant).
-template <int NT, int MINB>
+// Launch variants: blocks of 128 threads, with or without the registers capped
+// for three resident blocks per SM (the caps for four and eight spill and were
+// never chosen).  Chosen once per process by timing.
+constexpr int kTmThreads = 128;
+int tm_full_blocks(const Geom &g) { return 2 * ((g.Vh + kTmThreads - 1) / kTmThreads); }
+
+template <int MINB>
 static void launch_variant(cvcb_lattice *L, double2 *out, const double2 *in, double a, double b,
-                           double c, bool g5out, const int *done) {
+                           double c, bool g5out, const int *done, const TmDot *dot) {
   const Geom &g = L->g;
-  const int blocks = 2 * ((g.Vh + NT - 1) / NT);  // both parities, interleaved
-  if (g5out)
-    k_tm_full_f64<true, NT, MINB><<<blocks, NT, 0, L->stream>>>(out, in, L->U64, g, a, b, c, done);
-  else
-    k_tm_full_f64<false, NT, MINB><<<blocks, NT, 0, L->stream>>>(out, in, L->U64, g, a, b, c, done);
+  const int blocks = tm_full_blocks(g);  // both parities, interleaved
+  auto kern = g5out ? (dot ? k_tm_full_f64<true, true, kTmThreads, MINB> : k_tm_full_f64<true, false, kTmThreads, MINB>)
+                    : (dot ? k_tm_full_f64<false, true, kTmThreads, MINB> : k_tm_full_f64<false, false, kTmThreads, MINB>);
+  kern<<<blocks, kTmThreads, 0, L->stream>>>(out, in, L->U64, g, a, b, c, done, dot ? *dot : TmDot{});
 }
 
 static int g_tm_variant = -1;
-int tm_full_variant() { return g_tm_variant; }
-void set_tm_full_variant(int v) { g_tm_variant = v; }
 
 static void launch_by_variant(int v, cvcb_lattice *L, double2 *out, const double2 *in, double a,
-                              double b, double c, bool g5out, const int *done) {
-  switch (v) {
-    case 1: launch_variant<128, 4>(L, out, in, a, b, c, g5out, done); break;
-    case 2: launch_variant<256, 2>(L, out, in, a, b, c, g5out, done); break;
-    case 3: launch_variant<64, 8>(L, out, in, a, b, c, g5out, done); break;
-    case 4: launch_variant<128, 1>(L, out, in, a, b, c, g5out, done); break;
-    default: launch_variant<128, 3>(L, out, in, a, b, c, g5out, done); break;
-  }
+                              double b, double c, bool g5out, const int *done, const TmDot *dot) {
+  if (v == 1)
+    launch_variant<1>(L, out, in, a, b, c, g5out, done, dot);
+  else
+    launch_variant<3>(L, out, in, a, b, c, g5out, done, dot);
 }
 
 int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, double b, double c,
-                   bool g5out, const int *done) {
+                   bool g5out, const int *done, const TmDot *dot) {
   if (g_tm_variant < 0) {
     // one-time choice: time each variant on this lattice (output to `out`,
     // which the real launch below overwrites)
@@ -117,10 +182,10 @@ int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, d
     CVCB_CUDA(cudaEventCreate(&e1));
     float best = 1e30f;
     int bestv = 0;
-    for (int v = 0; v < 5; ++v) {
-      launch_by_variant(v, L, out, in, a, b, c, g5out, nullptr);
+    for (int v = 0; v < 2; ++v) {
+      launch_by_variant(v, L, out, in, a, b, c, g5out, nullptr, nullptr);
       CVCB_CUDA(cudaEventRecord(e0, L->stream));
-      for (int k = 0; k < 5; ++k) launch_by_variant(v, L, out, in, a, b, c, g5out, nullptr);
+      for (int k = 0; k < 5; ++k) launch_by_variant(v, L, out, in, a, b, c, g5out, nullptr, nullptr);
       CVCB_CUDA(cudaEventRecord(e1, L->stream));
       CVCB_CUDA(cudaEventSynchronize(e1));
       float ms;
@@ -134,7 +199,7 @@ int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, d
     cudaEventDestroy(e1);
     g_tm_variant = bestv;
   }
-  launch_by_variant(g_tm_variant, L, out, in, a, b, c, g5out, done);
+  launch_by_variant(g_tm_variant, L, out, in, a, b, c, g5out, done, dot);
   CVCB_LAUNCHED(L);
   return CVCB_OK;
 }

@@ -4,7 +4,8 @@
 // then x = Qf5(-mu) y, invert_Qtm.c:276-478).
 //
 // The recursion scalars live on the device (SolverScalars): the last block of
-// each reduction computes alpha, omega, beta and the convergence flag, and
+// each reduction computes alpha, omega, beta and the convergence flag
+// (bicgstab.cuh; alpha and omega in the operator sweeps themselves), and
 // every later kernel of the iteration reads them from HBM.  An iteration thus
 // costs no host round trip; the host checks the flag once per chunk of
 // iterations.  Once the flag is set, all remaining kernels of the chunk
@@ -13,43 +14,13 @@
 #include <algorithm>
 #include <cmath>
 
+#include "bicgstab.cuh"
 #include "cvcb_internal.h"
 #include "reduce.cuh"
 
 namespace cvcb {
 
 namespace {
-
-__device__ __forceinline__ double2 c_div(double2 a, double2 b) {
-  // _co_eq_co_ti_co_inv (cvc_complex.h): a / b = a conj(b) / |b|^2
-  const double n = b.x * b.x + b.y * b.y;
-  return make_double2((a.x * b.x + a.y * b.y) / n, (a.y * b.x - a.x * b.y) / n);
-}
-__device__ __forceinline__ double2 c_mul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ bool finite2(double2 a) { return isfinite(a.x) && isfinite(a.y); }
-
-// rho = <r2, r1>, w = <r2, p2>; alpha = rho / w  (invert_Qtm.c:161-163)
-struct RedRhoW {
-  const double2 *r2, *r1, *p2;
-  __device__ void operator()(size_t k, double (&acc)[4]) const {
-    const double2 a = __ldg(r2 + k), b = __ldg(r1 + k), c = __ldg(p2 + k);
-    acc[0] += a.x * b.x + a.y * b.y;
-    acc[1] += a.x * b.y - a.y * b.x;
-    acc[2] += a.x * c.x + a.y * c.y;
-    acc[3] += a.x * c.y - a.y * c.x;
-  }
-};
-struct EpiAlpha {
-  SolverScalars *S;
-  __device__ void operator()(const double (&t)[4]) const {
-    S->rho = make_double2(t[0], t[1]);
-    S->w = make_double2(t[2], t[3]);
-    S->alpha = c_div(S->rho, S->w);
-    if (!finite2(S->alpha)) { S->done = 2; S->niter = S->iter; }
-  }
-};
 
 // s = r1 - alpha p2   (invert_Qtm.c:171-176)
 __global__ void k_s_update(double2 *__restrict__ s, const double2 *__restrict__ r1,
@@ -65,97 +36,50 @@ __global__ void k_s_update(double2 *__restrict__ s, const double2 *__restrict__ 
   }
 }
 
-// w = <t, s>, u = <t, t>; omega = w / u  (invert_Qtm.c:182-184)
-struct RedOmega {
-  const double2 *t, *s;
-  __device__ void operator()(size_t k, double (&acc)[3]) const {
-    const double2 a = __ldg(t + k), b = __ldg(s + k);
-    acc[0] += a.x * b.x + a.y * b.y;
-    acc[1] += a.x * b.y - a.y * b.x;
-    acc[2] += a.x * a.x + a.y * a.y;
-  }
-};
-struct EpiOmega {
-  SolverScalars *S;
-  __device__ void operator()(const double (&t)[3]) const {
-    S->u = t[2];
-    // invert_Qtm.c:184 writes _co_eq_co_ti_re(&omega, &w, 1./u); the macro
-    // argument is not parenthesised, so it evaluates w.re*1./u = w.re / u.
-    S->omega = make_double2(t[0] / S->u, t[1] / S->u);
-    if (!finite2(S->omega)) { S->done = 2; S->niter = S->iter; }
-  }
-};
-
-// r1 = s - omega t; norm = <r1, r1>; stop if norm <= prec * normb
-// (invert_Qtm.c:192-201).
-struct RedR1 {
+// r1 = s - omega t; norm = <r1, r1>, w = <r2, r1>  (invert_Qtm.c:192-216)
+struct RedR1Beta {
   double2 *r1;
-  const double2 *s, *t;
+  const double2 *s, *t, *r2;
   const SolverScalars *S;
-  __device__ void operator()(size_t k, double (&acc)[1]) const {
+  __device__ void operator()(size_t k, double (&acc)[3]) const {
     const double2 q = c_mul(__ldg(t + k), S->omega);
-    const double2 a = __ldg(s + k);
+    const double2 a = __ldg(s + k), u = __ldg(r2 + k);
     const double2 r = make_double2(a.x - q.x, a.y - q.y);
     r1[k] = r;
     acc[0] += r.x * r.x + r.y * r.y;
+    acc[1] += u.x * r.x + u.y * r.y;
+    acc[2] += u.x * r.y - u.y * r.x;
   }
 };
-struct EpiNorm {
+struct EpiNormBeta {
   SolverScalars *S;
-  __device__ void operator()(const double (&t)[1]) const {
-    S->norm = t[0];
-    if (S->norm <= S->prec * S->normb) {
-      S->done = 1;
-      S->niter = S->iter;
-    } else if (!isfinite(S->norm)) {
-      S->done = 2;
-      S->niter = S->iter;
-    }
+  __device__ void operator()(const double (&t)[3]) const {
+    epi_norm_beta(S, t[0], make_double2(t[1], t[2]));
   }
 };
 
-// x += omega s + alpha p; w = <r2, r1>; beta = (w / rho)(alpha / omega);
-// rho = w  (invert_Qtm.c:204-218).  Skipped once converged: the reference
-// leaves the loop before this update.
-struct RedXBeta {
-  double2 *x;
-  const double2 *s, *p, *r2, *r1;
-  const SolverScalars *S;
-  __device__ void operator()(size_t k, double (&acc)[2]) const {
-    double2 xv = x[k];
-    const double2 a = c_mul(__ldg(s + k), S->omega);
-    xv.x += a.x; xv.y += a.y;
-    const double2 b = c_mul(__ldg(p + k), S->alpha);
-    xv.x += b.x; xv.y += b.y;
-    x[k] = xv;
-    const double2 u = __ldg(r2 + k), v = __ldg(r1 + k);
-    acc[0] += u.x * v.x + u.y * v.y;
-    acc[1] += u.x * v.y - u.y * v.x;
-  }
-};
-struct EpiBeta {
-  SolverScalars *S;
-  __device__ void operator()(const double (&t)[2]) const {
-    const double2 w = make_double2(t[0], t[1]);
-    const double2 w2 = c_div(w, S->rho);
-    const double2 w3 = c_div(S->alpha, S->omega);
-    S->beta = c_mul(w2, w3);
-    S->rho = w;
-    S->iter += 1;
-    if (!finite2(S->beta)) { S->done = 2; S->niter = S->iter; }
-  }
-};
-
-// p = r1 + beta (p - omega p2)  (invert_Qtm.c:224-231)
-__global__ void k_p_update(double2 *__restrict__ p, const double2 *__restrict__ r1,
-                           const double2 *__restrict__ p2, const SolverScalars *__restrict__ S,
-                           size_t n) {
-  if (S->done) return;
-  const double2 om = S->omega, be = S->beta;
+// x += omega s + alpha p (invert_Qtm.c:204-211) and p = r1 + beta (p - omega
+// p2) (:224-231) of iteration `iter`.  Skipped once converged: the reference
+// leaves the loop before the update of x; a beta that is not finite still
+// lets x take its step.
+__global__ void k_xp_update(double2 *__restrict__ x, double2 *__restrict__ p,
+                            const double2 *__restrict__ s, const double2 *__restrict__ r1,
+                            const double2 *__restrict__ p2, const SolverScalars *__restrict__ S,
+                            int iter, size_t n) {
+  if (S->done && S->xlast != iter) return;
+  const bool go = !S->done;
+  const double2 al = S->alpha, om = S->omega, be = S->beta;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
        k += (size_t)gridDim.x * blockDim.x) {
-    const double2 q = c_mul(__ldg(p2 + k), om);
     const double2 pv = p[k];
+    double2 xv = x[k];
+    const double2 a = c_mul(__ldg(s + k), om);
+    xv.x += a.x; xv.y += a.y;
+    const double2 b = c_mul(pv, al);
+    xv.x += b.x; xv.y += b.y;
+    x[k] = xv;
+    if (!go) continue;
+    const double2 q = c_mul(__ldg(p2 + k), om);
     const double2 d = make_double2(pv.x - q.x, pv.y - q.y);
     const double2 e = c_mul(d, be);
     const double2 r = __ldg(r1 + k);
@@ -189,6 +113,7 @@ struct EpiStart {
   SolverScalars *S;
   __device__ void operator()(const double (&t)[1]) const {
     S->norm = t[0];
+    S->rho = make_double2(t[0], 0.0);  // <r2, r1> with r1 = r2 = p
     if (S->norm <= S->prec * S->normb) { S->done = 3; S->niter = 0; }
   }
 };
@@ -202,11 +127,11 @@ int elem_blocks(size_t n) {
 
 // The operator of each solver on device-layout FP64 fields.
 static int apply_op(cvcb_lattice *L, bool her, double2 *out, const double2 *in, double2 *aux,
-                    const int *done) {
+                    const int *done, const TmDot *dot = nullptr) {
   const double a = 0.5 / L->kappa;
-  if (!her) return launch_tm_full(L, out, in, a, L->mu, -0.5, false, done);
-  CVCB_TRY(launch_tm_full(L, aux, in, a, -L->mu, -0.5, true, done));  // Qf5(aux, in, -mu)
-  return launch_tm_full(L, out, aux, a, L->mu, -0.5, true, done);     // Qf5(out, aux, +mu)
+  if (!her) return launch_tm_full(L, out, in, a, L->mu, -0.5, false, done, dot);
+  CVCB_TRY(launch_tm_full(L, aux, in, a, -L->mu, -0.5, true, done));    // Qf5(aux, in, -mu)
+  return launch_tm_full(L, out, aux, a, L->mu, -0.5, true, done, dot);  // Qf5(out, aux, +mu)
 }
 
 int invert_bicgstab(cvcb_lattice *L, bool her, double *xi, const double *phi, double prec,
@@ -215,18 +140,24 @@ int invert_bicgstab(cvcb_lattice *L, bool her, double *xi, const double *phi, do
   const size_t n = (size_t)g.V * 12;
   const size_t fb = n * sizeof(double2);
   void *base;
-  CVCB_TRY(ensure_buffer(L, SLOT_F2, 10 * fb, &base));
+  CVCB_TRY(ensure_buffer(L, SLOT_F2, 10 * fb + (size_t)tm_full_blocks(g) * 3 * sizeof(double), &base));
   double2 *F = static_cast<double2 *>(base);
   double2 *x = F, *rhs = F + n, *r1 = F + 2 * n, *r2 = F + 3 * n, *s = F + 4 * n,
           *t = F + 5 * n, *p = F + 6 * n, *p2 = F + 7 * n, *aux = F + 8 * n, *phid = F + 9 * n;
   SolverScalars *S = L->scal;
   const int eb = elem_blocks(n);
+  double *part = reinterpret_cast<double *>(F + 10 * n);
+  // alpha from <r2, p2> with the sweep that writes p2, omega from <t, s> and
+  // <t, t> with the one that writes t
+  const TmDot dot_alpha{1, r2, part, L->red_counter, S}, dot_omega{2, s, part, L->red_counter, S};
 
   CVCB_TRY(spinor_in(L, phid, phi, g.V));
   CVCB_TRY(spinor_in(L, x, xi, g.V));
 
   SolverScalars h{};
   h.prec = prec;
+  h.itmax = niter_max;
+  h.xlast = -1;
   CVCB_CUDA(cudaMemcpyAsync(S, &h, sizeof h, cudaMemcpyHostToDevice, L->stream));
 
   // normb = <phi, phi>  (invert_Qtm.c:129 / :329)
@@ -254,7 +185,7 @@ int invert_bicgstab(cvcb_lattice *L, bool her, double *xi, const double *phi, do
 
   CVCB_CUDA(cudaMemcpyAsync(r1, p, fb, cudaMemcpyDeviceToDevice, L->stream));
   CVCB_CUDA(cudaMemcpyAsync(r2, p, fb, cudaMemcpyDeviceToDevice, L->stream));
-  CVCB_TRY(apply_op(L, her, p2, p, aux, nullptr));
+  CVCB_TRY(apply_op(L, her, p2, p, aux, nullptr, &dot_alpha));
 
   const int *done = &S->done;
   const int chunk = 16;
@@ -262,16 +193,13 @@ int invert_bicgstab(cvcb_lattice *L, bool her, double *xi, const double *phi, do
   for (;;) {
     const int todo = std::min(chunk, niter_max + 1 - launched);
     for (int it = 0; it < todo; ++it) {
-      CVCB_TRY(launch_reduce<4>(L, RedRhoW{r2, r1, p2}, EpiAlpha{S}, n, done));
       k_s_update<<<eb, 256, 0, L->stream>>>(s, r1, p2, S, n);
       CVCB_LAUNCHED(L);
-      CVCB_TRY(apply_op(L, her, t, s, aux, done));
-      CVCB_TRY(launch_reduce<3>(L, RedOmega{t, s}, EpiOmega{S}, n, done));
-      CVCB_TRY(launch_reduce<1>(L, RedR1{r1, s, t, S}, EpiNorm{S}, n, done));
-      CVCB_TRY(launch_reduce<2>(L, RedXBeta{x, s, p, r2, r1, S}, EpiBeta{S}, n, done));
-      k_p_update<<<eb, 256, 0, L->stream>>>(p, r1, p2, S, n);
+      CVCB_TRY(apply_op(L, her, t, s, aux, done, &dot_omega));
+      CVCB_TRY(launch_reduce<3>(L, RedR1Beta{r1, s, t, r2, S}, EpiNormBeta{S}, n, done));
+      k_xp_update<<<eb, 256, 0, L->stream>>>(x, p, s, r1, p2, S, launched + it + 1, n);
       CVCB_LAUNCHED(L);
-      CVCB_TRY(apply_op(L, her, p2, p, aux, done));
+      CVCB_TRY(apply_op(L, her, p2, p, aux, done, &dot_alpha));
     }
     launched += todo;
     CVCB_CUDA(cudaMemcpyAsync(&hs, S, sizeof hs, cudaMemcpyDeviceToHost, L->stream));
