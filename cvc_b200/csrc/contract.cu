@@ -26,6 +26,7 @@
 // kernels of the path, which want the columns of all nu in the coefficient
 // form, k_cvc_z_sites or k_cvc_z builds the 24 columns
 // Z_c(x) = sum_{g,ib} conj(k us) chi_{d(g,ir,ib)}(x) of one nu.)
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -101,33 +102,45 @@ __global__ void __launch_bounds__(kZThreads) k_cvc_z_sites(double2 *__restrict__
 }
 
 // ---- the contraction kernel ------------------------------------------------
-// A block takes 8 consecutive lexicographic sites (V is a multiple of 16).
-// Per part it stages in shared memory the Z columns of all four nu (2 x 3
-// columns each, formed from the 48 shifted columns, every element read once
-// and coalesced although the fields are site-major) and the projected and
-// transported half spinors u of the 12 columns of the source point for the 8
-// neighbours; then each thread (colour of the sink, pair of nu with the same
-// spin partners, site, a, sign of the hop) forms its dots.  u is formed once
+// One block per SM walks through groups of 8 consecutive lexicographic sites
+// (V is a multiple of 16), two stages (parts) per group.  A stage forms in
+// shared memory the Z columns of all four nu (2 x 3 columns each) from the 48
+// shifted columns, and the projected and transported half spinors u of the 12
+// columns of the source point for the 8 neighbours; then each thread (colour
+// of the sink, nu, site, a, sign of the hop) forms its dots.  u is formed once
 // for all four nu, and the local columns need neither a copy in another
 // layout nor Z columns in memory.
+//
+// The SM holds only 12 warps of this (registers, shared memory), so a stage's
+// shifted columns (site-major, read once and coalesced) come to shared memory
+// by cp.async during the stage before, and so do the next group's links; the
+// first of a warp's two neighbour tasks is loaded into registers before the
+// dots of the stage before, the second before the Z columns are formed.
+//
 // Bounds at 24^3 x 48: 15.9 GB of compulsory traffic (2.4 ms at 6.55 TB/s) and
 // 42.6 k FP64 instructions per site (1.5 ms at 64 per SM and clock).  Measured
-// 7.5 ms (the whole contraction 9.2 ms; 44.6 ms with the columns copied to
-// component-major order, Z columns in memory and one thread per site; 0.27
-// against 2.41 ms at 8^3 x 16): load latency between the barriers at 12 warps
-// per SM bounds it (FP64 pipe 22 % busy).  Tried, no faster: all of a part's
-// local loads in flight at once and the links kept in registers (9.4 and
-// 9.7 ms), and bringing the next block's local columns to L2 (10.1 ms, DRAM
-// reads 1.5 times as many).
+// 7.1 ms (the whole contraction 8.3 ms; 44.6 ms with the columns copied to
+// component-major order, Z columns in memory and one thread per site; 0.26
+// against 2.41 ms at 8^3 x 16).  The shared-memory and load queues bound it
+// (L1 data pipe 51 %, FP64 pipe 21 % busy).  Measured against it: two blocks
+// of 6 warps without the asynchronous copies 8.8 ms, of 12 warps at 80
+// registers 9.7; one nu and all mu per thread, half again the reads of u, 8.6;
+// the source point's columns not tiled (below) 8.5; the shifted columns by
+// bulk copies 9.3; both neighbour tasks in flight together 11.4; another
+// order of the groups, with the neighbours' timeslices in L2, no change.
 constexpr int kPiSites = 8;
-constexpr int kPiThreads = 192;
-constexpr int kPiZ = 4 * 2 * 3 * 12 * kPiSites;  // double2: [nu][a][o][comp][site]
+constexpr int kPiThreads = 384, kPiWarps = kPiThreads / 32;
+constexpr int kPiZPitch = 13;                    // components of a site and one to spread the banks
+constexpr int kPiZ = 4 * 2 * 3 * kPiZPitch * kPiSites;  // double2: [nu][a][o][site][comp]
 constexpr int kPiU = 3 * 4 * 8 * 6 * kPiSites;   // double2: [ia][ir][dir][spin][colour][site]
-constexpr size_t kPiSmem = (kPiZ + kPiU) * sizeof(double2);
+constexpr int kPiRaw = 48 * 12 * kPiSites;       // double2: [column][site][comp]
+constexpr int kPiRed = 3 * 8 * 4 * kPiSites;     // double2: [sink colour][dir][nu][site]
+constexpr int kPiW = 8 * 9 * kPiSites;           // double2: [dir][entry][site], of this and the next group
+constexpr size_t kPiSmem = (kPiZ + kPiU + kPiRaw + kPiRed + 2 * kPiW) * sizeof(double2);
 
 struct PiArgs {
   const double2 *loc[2][48];  // part 0: dn, part 1: up columns of the shifted points, site-major
-  const double2 *fix;         // [part][12 columns][12][V], lexicographic: columns of the source point
+  const double2 *fix;         // columns of the source point (fix_slot)
   const double2 *U;
   double2 *F, *B;   // T_+ and T_-, [V][mu][nu]
   double2 us[4][9]; // conj of the phased source links
@@ -135,26 +148,63 @@ struct PiArgs {
   Geom g;
 };
 
-// slot of component comp of site s inside one Z column: the sites of a
-// component are permuted by it, so that both the writers (consecutive
-// components) and the readers (consecutive sites) spread over the banks
-__device__ __forceinline__ int z_slot(int comp, int s) { return comp * kPiSites + (s ^ (comp & 7)); }
+__device__ __forceinline__ SiteCoord lex_coord(const Geom &g, int lex) {
+  SiteCoord cd;
+  const unsigned r0 = fdiv((unsigned)lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
+  cd.lex = lex;
+  cd.z = lex - (int)r0 * g.LZ;
+  cd.y = (int)(r0 - r1 * g.LY);
+  cd.x = (int)(r1 - r2 * g.LX);
+  cd.t = (int)r2;
+  return cd;
+}
 
-// u of one column and direction for the thread's site
-template <int MU, int S>
-__device__ __forceinline__ void pi_transport(const PiArgs &A, const SiteCoord &cd, int par,
-                                             const double2 *col, double2 *u) {
+// Columns of the source point, tiled by 8 lexicographic sites with all 24
+// columns (12 up, 12 dn) of a tile together: [tile][column][component][site].
+// A group's neighbours in one direction are then one or two runs of 37 KB;
+// with the columns apart, every 128 bytes came from another page.
+__device__ __forceinline__ size_t fix_slot(int lex, int col) {
+  return ((size_t)(lex >> 3) * 24 + col) * 12 * kPiSites + (lex & 7);
+}
+
+__device__ __forceinline__ void cp_async16(double2 *dst, const double2 *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+
+// the 64 links of a group's hops: dir = mu (forward, at the site) or 4 + mu
+// (backward, at the neighbour)
+__device__ __forceinline__ void pi_fetch_links(const PiArgs &A, double2 *sw, int base) {
   const Geom &g = A.g;
-  const int j = nb_lex(g, cd, MU, S < 0 ? +1 : -1);
+  for (int k = threadIdx.x; k < kPiW; k += kPiThreads) {
+    const int site = k % kPiSites, q = k / kPiSites, e = q % 9, dir = q / 9, mu = dir & 3;
+    const SiteCoord cd = lex_coord(g, base + site);
+    const int par = (cd.t + cd.x + cd.y + cd.z) & 1;
+    const int at = dir < 4 ? par * g.Vh + (cd.lex >> 1) : (1 - par) * g.Vh + (nb_lex(g, cd, mu, -1) >> 1);
+    cp_async16(sw + k, A.U + (size_t)(mu * 9 + e) * g.V + at);
+  }
+}
+
+// One neighbour task q = 3 direction + colour: the column of the lane's source
+// spin at the neighbour of the lane's site.
+__device__ __forceinline__ void pi_load(double2 (&f)[12], const PiArgs &A, int lex, int part, int q, int ir) {
+  const Geom &g = A.g;
+  const int j = nb_lex(g, lex_coord(g, lex), q / 3 & 3, q < 12 ? +1 : -1);
+  const double2 *col = A.fix + fix_slot(j, part * 12 + 3 * ir + q % 3);
+#pragma unroll
+  for (int k = 0; k < 12; ++k) f[k] = __ldg(col + k * kPiSites);
+}
+template <int MU, int S>
+__device__ __forceinline__ void pi_transport(const double2 (&fv)[12], const double2 *w, double2 *u) {
   Spinor<double> f;
 #pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    const double2 v = __ldg(col + (size_t)k * g.V + j);
-    f.c[k / 3][k % 3] = cx(v.x, v.y);
-  }
-  const int at = S < 0 ? par * g.Vh + (cd.lex >> 1) : (1 - par) * g.Vh + (j >> 1);
-  const Link<double> W = load_link64(A.U, g.V, MU, at);
+  for (int k = 0; k < 12; ++k) f.c[k / 3][k % 3] = cx(fv[k].x, fv[k].y);
   const HalfSpinor<double> h = project(MU, S, f);
+  Link<double> W;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) W.m[k / 3][k % 3] = cx(w[k * kPiSites].x, w[k * kPiSites].y);
   const HalfSpinor<double> r = S < 0 ? link_mul(W, h) : link_dag_mul(W, h);
 #pragma unroll
   for (int b = 0; b < 2; ++b)
@@ -162,11 +212,23 @@ __device__ __forceinline__ void pi_transport(const PiArgs &A, const SiteCoord &c
     for (int c = 0; c < 3; ++c)
       u[(3 * b + c) * kPiSites] = make_double2(r.c[b][c].re, r.c[b][c].im);
 }
-
-// acc += conj(z) v
-__device__ __forceinline__ void dot_acc(Cx<double> &acc, Cx<double> z, Cx<double> v) {
-  cfmac(acc, z, v);
+__device__ __forceinline__ void pi_store(const double2 (&f)[12], const double2 *sw, double2 *su, int q,
+                                         int ir, int site) {
+  const int dir = q / 3, ia = q % 3;
+  double2 *u = su + ((ia * 4 + ir) * 8 + dir) * 6 * kPiSites + site;
+  const double2 *w = sw + dir * 9 * kPiSites + site;
+  switch (dir) {
+    case 0: pi_transport<0, -1>(f, w, u); break;
+    case 1: pi_transport<1, -1>(f, w, u); break;
+    case 2: pi_transport<2, -1>(f, w, u); break;
+    case 3: pi_transport<3, -1>(f, w, u); break;
+    case 4: pi_transport<0, +1>(f, w, u); break;
+    case 5: pi_transport<1, +1>(f, w, u); break;
+    case 6: pi_transport<2, +1>(f, w, u); break;
+    default: pi_transport<3, +1>(f, w, u); break;
+  }
 }
+
 // z + s w and z + s i w
 __device__ __forceinline__ Cx<double> add_s(Cx<double> z, double s, Cx<double> w) {
   return cx(fma(s, w.re, z.re), fma(s, w.im, z.im));
@@ -175,133 +237,143 @@ __device__ __forceinline__ Cx<double> add_si(Cx<double> z, double s, Cx<double> 
   return cx(fma(-s, w.im, z.re), fma(s, w.re, z.im));
 }
 
-__global__ void __launch_bounds__(kPiThreads, 2) k_pi(const __grid_constant__ PiArgs A) {
-  extern __shared__ double2 sm[];
-  double2 *sz = sm, *su = sm + kPiZ;
-  const Geom &g = A.g;
-  const int base = blockIdx.x * kPiSites;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int site = lane & 7;
-  SiteCoord cd;
-  {
-    cd.lex = base + site;
-    const unsigned r0 = fdiv((unsigned)cd.lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
-    cd.z = cd.lex - (int)r0 * g.LZ;
-    cd.y = (int)(r0 - r1 * g.LY);
-    cd.x = (int)(r1 - r2 * g.LX);
-    cd.t = (int)r2;
+// a stage's 48 local columns of the 8 sites from lexicographic site `base`
+__device__ __forceinline__ void pi_fetch_local(const PiArgs &A, double2 *raw, int base, int part) {
+  for (int k = threadIdx.x; k < kPiRaw; k += kPiThreads) {
+    const int col = k / (12 * kPiSites), e = k % (12 * kPiSites);
+    cp_async16(raw + k, A.loc[part][col] + (size_t)base * 12 + e);
   }
-  const int par = (cd.t + cd.x + cd.y + cd.z) & 1;
-  // the dots' role of the thread
-  const int si = warp % 3, cls = warp / 3;           // colour of the sink; nu in {0,3} or {2,1}
-  const int a = (lane >> 3) & 1, sg = lane >> 4;     // source spin; forward or backward hop
-  const int ap = cls == 0 ? a + 2 : 3 - a;           // its partner
-  const int nur = cls == 0 ? 0 : 2, nui = cls == 0 ? 3 : 1;
-  const double lr = A.lam[nur][a], li = A.lam[nui][a];
-  const double s = sg ? 1.0 : -1.0;
-  Cx<double> acc[2][4];
-#pragma unroll
-  for (int n = 0; n < 2; ++n)
-#pragma unroll
-    for (int mu = 0; mu < 4; ++mu) acc[n][mu] = cx(0.0, 0.0);
+}
 
+// Z columns: 8 (nu, a) x 96 elements (site, component), six columns in, three out
+__device__ __forceinline__ void pi_z(const PiArgs &A, double2 *sz, const double2 *raw, int warp, int lane) {
 #pragma unroll 1
-  for (int part = 0; part < 2; ++part) {
-    // Z: 8 (nu, a) x 96 elements (site, component), six columns in, three out
-#pragma unroll 1
-    for (int q = warp; q < 24; q += kPiThreads / 32) {
-      const int na = q / 3, nu = na >> 1, za = na & 1;
-      const int zp = nu == 0 || nu == 3 ? za + 2 : 3 - za;
-      const int e = (q % 3) * 32 + lane, es = e / 12, ec = e - 12 * es;
-      const size_t off = (size_t)base * 12 + e;
-      const double l = A.lam[nu][za];
-      Cx<double> y[3];
+  for (int q = warp; q < 24; q += kPiWarps) {
+    const int na = q / 3, nu = na >> 1, za = na & 1;
+    const int zp = nu == 0 || nu == 3 ? za + 2 : 3 - za;
+    const int e = (q % 3) * 32 + lane, es = e / 12, ec = e - 12 * es;
+    const double2 *f = raw + 12 * nu * 12 * kPiSites + e;
+    const double l = A.lam[nu][za];
+    Cx<double> y[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const double2 v = __ldg(A.loc[part][12 * nu + 3 * za + i] + off);
-        const double2 w = __ldg(A.loc[part][12 * nu + 3 * zp + i] + off);
-        y[i] = nu & 1 ? add_si(cx(v.x, v.y), -l, cx(w.x, w.y)) : add_s(cx(v.x, v.y), -l, cx(w.x, w.y));
-      }
-#pragma unroll
-      for (int o = 0; o < 3; ++o) {
-        Cx<double> z = cx(0.0, 0.0);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) cfma(z, cx(A.us[nu][3 * o + i].x, A.us[nu][3 * o + i].y), y[i]);
-        sz[(na * 3 + o) * 12 * kPiSites + z_slot(ec, es)] = make_double2(z.re, z.im);
-      }
+    for (int i = 0; i < 3; ++i) {
+      const double2 v = f[(3 * za + i) * 12 * kPiSites], w = f[(3 * zp + i) * 12 * kPiSites];
+      y[i] = nu & 1 ? add_si(cx(v.x, v.y), -l, cx(w.x, w.y)) : add_s(cx(v.x, v.y), -l, cx(w.x, w.y));
     }
-    // u: 8 directions x 3 colours, lanes = 8 sites x 4 source spins
-#pragma unroll 1
-    for (int q = warp; q < 24; q += kPiThreads / 32) {
-      const int dir = q / 3, ia = q % 3, ir = lane >> 3;
-      const double2 *col = A.fix + (size_t)(part * 12 + 3 * ir + ia) * 12 * g.V;
-      double2 *u = su + ((ia * 4 + ir) * 8 + dir) * 6 * kPiSites + site;
-      switch (dir) {
-        case 0: pi_transport<0, -1>(A, cd, par, col, u); break;
-        case 1: pi_transport<1, -1>(A, cd, par, col, u); break;
-        case 2: pi_transport<2, -1>(A, cd, par, col, u); break;
-        case 3: pi_transport<3, -1>(A, cd, par, col, u); break;
-        case 4: pi_transport<0, +1>(A, cd, par, col, u); break;
-        case 5: pi_transport<1, +1>(A, cd, par, col, u); break;
-        case 6: pi_transport<2, +1>(A, cd, par, col, u); break;
-        default: pi_transport<3, +1>(A, cd, par, col, u); break;
-      }
-    }
-    __syncthreads();
-#pragma unroll 1
+#pragma unroll
     for (int o = 0; o < 3; ++o) {
-      Cx<double> zr[4], zi[4];
+      Cx<double> z = cx(0.0, 0.0);
 #pragma unroll
-      for (int sp = 0; sp < 4; ++sp) {
-        const int sl = z_slot(3 * sp + si, site);
-        const double2 v = sz[((nur * 2 + a) * 3 + o) * 12 * kPiSites + sl];
-        const double2 w = sz[((nui * 2 + a) * 3 + o) * 12 * kPiSites + sl];
-        zr[sp] = cx(v.x, v.y);
-        zi[sp] = cx(w.x, w.y);
-      }
+      for (int i = 0; i < 3; ++i) cfma(z, cx(A.us[nu][3 * o + i].x, A.us[nu][3 * o + i].y), y[i]);
+      sz[((na * 3 + o) * kPiSites + es) * kPiZPitch + ec] = make_double2(z.re, z.im);
+    }
+  }
+}
+
+// The dots of one thread: both nu of a class (zr with a real lam, zi with an
+// imaginary one: they share the u that they read) and mu = 2 MH, 2 MH + 1.
+template <int MH>
+__device__ __forceinline__ void pi_dots(Cx<double> (&acc)[2][2], const double2 *zr, const double2 *zi,
+                                        const double2 *su, double lr, double li, double s, int si,
+                                        int site, int a, int ap, int sg) {
+#pragma unroll 1
+  for (int o = 0; o < 3; ++o) {
+    Cx<double> z[2][4];
 #pragma unroll
-      for (int mu = 0; mu < 4; ++mu) {
-        const int d = sg * 4 + mu;
-        const double2 *u1 = su + (((o * 4 + a) * 8 + d) * 6 + si) * kPiSites + site;
-        const double2 *u2 = su + (((o * 4 + ap) * 8 + d) * 6 + si) * kPiSites + site;
+    for (int sp = 0; sp < 4; ++sp) {
+      const int k = (o * kPiSites + site) * kPiZPitch + 3 * sp + si;
+      z[0][sp] = cx(zr[k].x, zr[k].y);
+      z[1][sp] = cx(zi[k].x, zi[k].y);
+    }
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const double2 p = u1[3 * b * kPiSites], q = u2[3 * b * kPiSites];
-          const Cx<double> vr = add_s(cx(p.x, p.y), lr, cx(q.x, q.y));
-          const Cx<double> vi = add_si(cx(p.x, p.y), li, cx(q.x, q.y));
-          // the conjugate-transposed reconstruction of spins 2, 3 with g5
-          const int hi = mu == 0 || mu == 3 ? 2 + b : 3 - b;
-          const double sb = (mu >= 2 && b == 1) ? -s : s;
-          const bool im = mu & 1;
-          dot_acc(acc[0][mu], im ? add_si(zr[b], sb, zr[hi]) : add_s(zr[b], sb, zr[hi]), vr);
-          dot_acc(acc[1][mu], im ? add_si(zi[b], sb, zi[hi]) : add_s(zi[b], sb, zi[hi]), vi);
-        }
+    for (int m = 0; m < 2; ++m) {
+      const int mu = 2 * MH + m, d = sg * 4 + mu;
+      const double2 *u1 = su + (((o * 4 + a) * 8 + d) * 6 + si) * kPiSites + site;
+      const double2 *u2 = su + (((o * 4 + ap) * 8 + d) * 6 + si) * kPiSites + site;
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const double2 p = u1[3 * b * kPiSites], q = u2[3 * b * kPiSites];
+        const Cx<double> vr = add_s(cx(p.x, p.y), lr, cx(q.x, q.y));
+        const Cx<double> vi = add_si(cx(p.x, p.y), li, cx(q.x, q.y));
+        // the conjugate-transposed reconstruction of spins 2, 3 with g5
+        const int hi = mu == 0 || mu == 3 ? 2 + b : 3 - b;
+        const double sb = (mu >= 2 && b == 1) ? -s : s;
+        cfmac(acc[0][m], (mu & 1) ? add_si(z[0][b], sb, z[0][hi]) : add_s(z[0][b], sb, z[0][hi]), vr);
+        cfmac(acc[1][m], (mu & 1) ? add_si(z[1][b], sb, z[1][hi]) : add_s(z[1][b], sb, z[1][hi]), vi);
       }
     }
-    __syncthreads();
-    // the second part enters conjugated: conj(conj(T_0) + T_1)
+  }
+}
+
+__global__ void __launch_bounds__(kPiThreads, 1) k_pi(const __grid_constant__ PiArgs A) {
+  extern __shared__ double2 sm[];
+  double2 *sz = sm, *su = sz + kPiZ, *raw = su + kPiU, *red = raw + kPiRaw, *sw = red + kPiRed;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int site = lane & 7, ir = lane >> 3;  // of the neighbour tasks
+  // the dots' role of the thread
+  const int si = warp % 3, cls = warp / 3 & 1, mh = warp / 6;  // colour of the sink; nu in {0,3} or {2,1}; mu
+  const int a = (lane >> 3) & 1, sg = lane >> 4;               // source spin; forward or backward hop
+  const int ap = cls == 0 ? a + 2 : 3 - a;                     // its partner
+  const int nur = cls == 0 ? 0 : 2, nui = cls == 0 ? 3 : 1;
+  const double lr = A.lam[nur][a], li = A.lam[nui][a], s = sg ? 1.0 : -1.0;
+  const double2 *zr = sz + (nur * 2 + a) * 3 * kPiSites * kPiZPitch;
+  const double2 *zi = sz + (nui * 2 + a) * 3 * kPiSites * kPiZPitch;
+  const int step = gridDim.x * kPiSites;
+  int base = blockIdx.x * kPiSites, wb = 0;  // wb: which half of sw holds this group's links
+  if (base >= A.g.V) return;
+  double2 f[12];
+  pi_fetch_local(A, raw, base, 0);
+  pi_fetch_links(A, sw, base);
+  pi_load(f, A, base + site, 0, warp, ir);
+  for (;; base += step, wb = kPiW - wb) {
+    Cx<double> acc[2][2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) acc[n][0] = acc[n][1] = cx(0.0, 0.0);
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();  // raw and the links are complete; the dots of the stage before are done
+      pi_store(f, sw + wb, su, warp, ir, site);
+      pi_load(f, A, base + site, part, warp + kPiWarps, ir);
+      pi_z(A, sz, raw, warp, lane);
+      pi_store(f, sw + wb, su, warp + kPiWarps, ir, site);
+      __syncthreads();  // sz and su are complete, raw is free
+      const int nbase = part ? base + step : base;  // the next stage
+      if (nbase < A.g.V) {
+        pi_fetch_local(A, raw, nbase, 1 - part);
+        if (part) pi_fetch_links(A, sw + (kPiW - wb), nbase);
+        pi_load(f, A, nbase + site, 1 - part, warp, ir);
+      }
+      if (mh)
+        pi_dots<1>(acc, zr, zi, su, lr, li, s, si, site, a, ap, sg);
+      else
+        pi_dots<0>(acc, zr, zi, su, lr, li, s, si, site, a, ap, sg);
+      // the second part enters conjugated: conj(conj(T_0) + T_1)
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) acc[n][m].im = -acc[n][m].im;
+    }
+    // sum over a (lanes) and the sink's colour (warps), in a fixed order
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int mu = 0; mu < 4; ++mu) acc[n][mu].im = -acc[n][mu].im;
-  }
-  // sum over a (lanes) and the sink's colour (warps), in a fixed order
-#pragma unroll
-  for (int n = 0; n < 2; ++n)
-#pragma unroll
-    for (int mu = 0; mu < 4; ++mu) {
-      Cx<double> t = acc[n][mu];
-      t.re += __shfl_xor_sync(0xffffffffu, t.re, 8);
-      t.im += __shfl_xor_sync(0xffffffffu, t.im, 8);
-      if (a == 0)
-        sm[((si * 8 + sg * 4 + mu) * 4 + (n ? nui : nur)) * kPiSites + site] = make_double2(t.re, t.im);
+      for (int m = 0; m < 2; ++m) {
+        Cx<double> v = acc[n][m];
+        v.re += __shfl_xor_sync(0xffffffffu, v.re, 8);
+        v.im += __shfl_xor_sync(0xffffffffu, v.im, 8);
+        if (a == 0)
+          red[((si * 8 + sg * 4 + 2 * mh + m) * 4 + (n ? nui : nur)) * kPiSites + site] = make_double2(v.re, v.im);
+      }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      const int k = threadIdx.x, ks = (k >> 4) & 7;
+      const int slot = (((k >> 7) * 4 + ((k >> 2) & 3)) * 4 + (k & 3)) * kPiSites + ks;
+      const double2 x = red[slot], y = red[slot + kPiRed / 3], w = red[slot + 2 * (kPiRed / 3)];
+      double2 *o = (k >> 7) ? A.B : A.F;
+      o[(size_t)(base + ks) * 16 + (k & 15)] = make_double2(x.x + y.x + w.x, x.y + y.y + w.y);
     }
-  __syncthreads();
-  for (int k = threadIdx.x; k < 256; k += kPiThreads) {
-    const int ks = (k >> 4) & 7, slot = (((k >> 7) * 4 + ((k >> 2) & 3)) * 4 + (k & 3)) * kPiSites + ks;
-    const double2 x = sm[slot], y = sm[slot + 32 * kPiSites], z = sm[slot + 64 * kPiSites];
-    double2 *o = (k >> 7) ? A.B : A.F;
-    o[(size_t)(base + ks) * 16 + (k & 15)] = make_double2(x.x + y.x + z.x, x.y + y.y + z.y);
+    if (base + step >= A.g.V) break;
   }
 }
 
@@ -310,20 +382,13 @@ __global__ void k_pi_combine(double2 *__restrict__ conn, const double2 *__restri
                              const double2 *__restrict__ B, Geom g) {
   const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (k >= (size_t)g.V * 16) return;
-  SiteCoord cd;
-  cd.lex = (int)(k >> 4);
-  const unsigned r0 = fdiv((unsigned)cd.lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
-  cd.z = cd.lex - (int)r0 * g.LZ;
-  cd.y = (int)(r0 - r1 * g.LY);
-  cd.x = (int)(r1 - r2 * g.LX);
-  cd.t = (int)r2;
+  const SiteCoord cd = lex_coord(g, (int)(k >> 4));
   const int m = (int)(k & 15);
   const double2 f = F[k], b = B[(size_t)nb_lex(g, cd, m >> 2, +1) * 16 + m];
   conn[k] = make_double2(-0.25 * (f.x - b.x), -0.25 * (f.y - b.y));
 }
 
-// columns of the source point from CVC layout to component-major:
-// dst[column][component][V], lexicographic
+// columns of the source point from CVC layout to the tiles of fix_slot
 struct FixCols {
   const double2 *src[24];
 };
@@ -333,15 +398,11 @@ __global__ void __launch_bounds__(128) k_fix_columns(double2 *__restrict__ dst,
   __shared__ double2 t[kFixTile * 13];
   const int base = blockIdx.x * kFixTile, n = min(kFixTile, V - base);
   const double2 *src = c.src[blockIdx.y] + (size_t)base * 12;
-  for (int q = threadIdx.x; q < n * 12; q += blockDim.x) {
-    const int s = q / 12;
-    t[q + s] = __ldg(src + q);
-  }
+  for (int q = threadIdx.x; q < n * 12; q += blockDim.x) t[q + q / 12] = __ldg(src + q);
   __syncthreads();
-  double2 *d = dst + (size_t)blockIdx.y * 12 * V + base;
-  for (int q = threadIdx.x; q < kFixTile * 12; q += blockDim.x) {
-    const int k = q / kFixTile, s = q % kFixTile;
-    if (s < n) d[(size_t)k * V + s] = t[s * 13 + k];
+  for (int q = threadIdx.x; q < n * 12; q += blockDim.x) {
+    const int tile = q / (12 * kPiSites), r = q % (12 * kPiSites), k = r / kPiSites, s = r % kPiSites;
+    dst[fix_slot(base + tile * kPiSites, blockIdx.y) + r] = t[(tile * kPiSites + s) * 13 + k];
   }
 }
 
@@ -662,7 +723,9 @@ int cvc_contract(cvcb_lattice *L, const double *const *fields, int src, double *
       static_cast<double2 *>(fixb), fc, g.V);
   CVCB_LAUNCHED(L);
   CVCB_CUDA(cudaFuncSetAttribute(k_pi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPiSmem));
-  k_pi<<<g.V / kPiSites, kPiThreads, kPiSmem, L->stream>>>(A);
+  int sms = 0;
+  CVCB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, L->device));
+  k_pi<<<std::min(g.V / kPiSites, sms), kPiThreads, kPiSmem, L->stream>>>(A);
   CVCB_LAUNCHED(L);
   // contact term (:697-704, :837-844) from a handful of spinors
   double *ctb = reinterpret_cast<double *>(A.B + piv);
