@@ -109,27 +109,74 @@ bool split_radix(int L, Radix *r) {
   return r->n1 != 0;
 }
 
+// cos and sin of 2 pi j / n for n <= 8, as constants of the unrolled transforms
+// (no registers for the roots, and no arithmetic for 0 and +-1)
+__host__ __device__ constexpr double root_cos(int n, int j) {
+  constexpr double c5[3] = {1.0, 0.30901699437494742410, -0.80901699437494742410};
+  constexpr double c7[4] = {1.0, 0.62348980185873353053, -0.22252093395631440429,
+                            -0.90096886790241912624};
+  constexpr double h = 0.70710678118654752440;
+  constexpr double c8[5] = {1.0, h, 0.0, -h, -1.0};
+  const int m = j > n - j ? n - j : j;  // cos is even about n / 2
+  return n == 5 ? c5[m] : n == 7 ? c7[m] : n == 8 ? c8[m] : n == 4 ? c8[2 * m]
+       : n == 2 ? c8[4 * m] : n == 1 ? 1.0
+       : (n == 3 ? 2 * m : m) == 0 ? 1.0 : (n == 3 ? 2 * m : m) == 1 ? 0.5
+       : (n == 3 ? 2 * m : m) == 2 ? -0.5 : -1.0;  // 3, 6
+}
+__host__ __device__ constexpr double root_sin(int n, int j) {
+  constexpr double s5[3] = {0.0, 0.95105651629515357212, 0.58778525229247312917};
+  constexpr double s7[4] = {0.0, 0.78183148246802980871, 0.97492791218182360702,
+                            0.43388373911755812048};
+  constexpr double h = 0.70710678118654752440, q = 0.86602540378443864676;
+  constexpr double s8[5] = {0.0, h, 1.0, h, 0.0};
+  const bool up = 2 * j > n;
+  const int m = up ? n - j : j;  // odd about n / 2
+  const double v = n == 5 ? s5[m] : n == 7 ? s7[m] : n == 8 ? s8[m] : n == 4 ? s8[2 * m]
+                 : n <= 2 ? 0.0
+                 : (n == 3 ? 2 * m : m) == 0 || (n == 3 ? 2 * m : m) == 3 ? 0.0 : q;
+  return up ? -v : v;
+}
+// (re, im) += e^{-2 pi i j / n} v, all but v known to the compiler
+__device__ __forceinline__ void add_root(double &re, double &im, int n, int j, double2 v) {
+  const double c = root_cos(n, j), s = -root_sin(n, j);
+  if (s == 0.0) {
+    re = c == 1.0 ? re + v.x : c == -1.0 ? re - v.x : fma(c, v.x, re);
+    im = c == 1.0 ? im + v.y : c == -1.0 ? im - v.y : fma(c, v.y, im);
+  } else if (c == 0.0) {
+    re = s == 1.0 ? re - v.y : re + v.y;
+    im = s == 1.0 ? im + v.x : im - v.x;
+  } else {
+    re = fma(-s, v.y, fma(c, v.x, re));
+    im = fma(s, v.x, fma(c, v.y, im));
+  }
+}
+
 // n values at p[k * stride] -> their transform, in place; roots[j * step] =
 // e^{-2 pi i j / n}; entry k is multiplied by tw[k * m] (tw null: not)
 template <int N>
 __device__ __forceinline__ void dft_reg(double2 *p, int stride, const double2 *roots, int step,
                                         const double2 *tw, int m) {
-  double2 v[N], w[N];
+  double2 v[N];
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    v[k] = p[k * stride];
-    w[k] = roots[k * step];
-  }
+  for (int k = 0; k < N; ++k) v[k] = p[k * stride];
+  double2 w[N > 8 ? N : 1];
+  if constexpr (N > 8)
+#pragma unroll
+    for (int k = 0; k < N; ++k) w[k] = roots[k * step];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     double re = v[0].x, im = v[0].y;
 #pragma unroll
     for (int x = 1; x < N; ++x) {
-      const double2 c = w[(x * k) % N];
-      re = fma(c.x, v[x].x, re);
-      re = fma(-c.y, v[x].y, re);
-      im = fma(c.x, v[x].y, im);
-      im = fma(c.y, v[x].x, im);
+      if constexpr (N > 8) {
+        const double2 c = w[(x * k) % N];
+        re = fma(c.x, v[x].x, re);
+        re = fma(-c.y, v[x].y, re);
+        im = fma(c.x, v[x].y, im);
+        im = fma(c.y, v[x].x, im);
+      } else {
+        add_root(re, im, N, (x * k) % N, v[x]);
+      }
     }
     if (tw) {
       const double2 c = tw[k * m];
@@ -188,14 +235,17 @@ __device__ __forceinline__ void dft_plane(double2 *sm, const double2 *tw, Radix 
 }
 
 // Two directions (a, b) of every plane.  Element (i, j) of plane o, entry c:
-// (i Lb + j) es + o os + c; a block takes the plane o = blockIdx.x and the nc
-// entries from nc * blockIdx.y.  P: midpoint phases on the way out (the
-// planes are then (t, x) and o = (y, z)).  MAXR: largest factor held in
-// registers; up to 8, which covers 2, 4, ... 16, 20, 24, 28, 30, 32, 36, 40,
-// 42, 48, 56, 64, two blocks fit an SM (larger ones need 236 registers).
+// (i Lb + j) es + o os + c; a block takes one plane o and nc of its 16 entries,
+// consecutive blocks the entries of one plane (they share its cache lines:
+// DRAM reads of the second launch 336 -> 170 MB).  phases: midpoint phases on
+// the way out (the planes are then (t, x) and o = (y, z)).  MAXR: largest
+// factor held in registers; up to 8, which covers 2, 4, ... 16, 20, 24, 28, 30,
+// 32, 36, 40, 42, 48, 56, 64, the roots are constants and three blocks fit an
+// SM (larger ones keep them in registers, 236 in all).
 // Moves 0.68 GB at 24^3 x 48 in the two launches, 0.10 ms at 6.55 TB/s;
-// measured 0.18 and 0.27 ms, issue-bound on index arithmetic and FP64 (2.85 ms
-// for the whole call with four k_dft_axis passes, a phase pass and two copies).
+// measured 0.13 and 0.22 ms (0.37 ms for the call), issue-bound on index
+// arithmetic and FP64; 2.85 ms with four k_dft_axis passes, a phase pass and
+// two copies.  With two blocks per SM 0.41 ms, with four 0.41 (spills).
 constexpr int kDftThreads = 256;
 constexpr size_t kDftSmem = 220 * 1024;
 struct DftPair {
@@ -206,12 +256,13 @@ struct DftPair {
   int lnc, phases;  // nc = 1 << lnc
 };
 template <int MAXR>
-__global__ void __launch_bounds__(kDftThreads, MAXR > 8 ? 1 : 2)
+__global__ void __launch_bounds__(kDftThreads, MAXR > 8 ? 1 : 3)
     k_dft_pair(const __grid_constant__ DftPair D, const __grid_constant__ PhaseArgs P) {
   extern __shared__ double2 sm[];
   const int La = D.a.L, Lb = D.b.L, nc = 1 << D.lnc, n = La * Lb * nc;
   double2 *ta = sm + n, *tb = ta + La;
-  const long long base = (long long)blockIdx.x * D.os + (long long)blockIdx.y * nc;
+  const int plane = blockIdx.x / (16 >> D.lnc), c0 = blockIdx.x % (16 >> D.lnc) * nc;
+  const long long base = plane * D.os + c0;
   for (int q = threadIdx.x; q < La + Lb; q += kDftThreads) ta[q] = q < La ? D.ta[q] : D.tb[q - La];
 #pragma unroll 4
   for (int q = threadIdx.x; q < n; q += kDftThreads)
@@ -226,7 +277,7 @@ __global__ void __launch_bounds__(kDftThreads, MAXR > 8 ? 1 : 2)
     const int sa = D.a.n2 * (ka - a2 * D.a.n1) + a2, sb = D.b.n2 * (kb - b2 * D.b.n1) + b2;
     double2 v = sm[((sa * Lb + sb) << D.lnc) + c];
     if (D.phases)
-      v = pi_phase(P, ka, kb, blockIdx.x / P.LZ, blockIdx.x % P.LZ, blockIdx.y * nc + c, v);
+      v = pi_phase(P, ka, kb, plane / P.LZ, plane % P.LZ, c0 + c, v);
     D.out[base + (q >> D.lnc) * D.es + c] = v;
   }
 }
@@ -245,7 +296,7 @@ int launch_dft_pair(cvcb_lattice *L, const DftPair &D, const PhaseArgs &P, long 
   auto kern = std::max(std::max(D.a.n1, D.a.n2), std::max(D.b.n1, D.b.n2)) <= 8 ? k_dft_pair<8>
                                                                                : k_dft_pair<kMaxRadix>;
   CVCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem));
-  kern<<<dim3((unsigned)planes, 16 >> D.lnc), kDftThreads,
+  kern<<<(unsigned)(planes * (16 >> D.lnc)), kDftThreads,
          (((size_t)D.a.L * D.b.L << D.lnc) + D.a.L + D.b.L) * sizeof(double2), L->stream>>>(D, P);
   CVCB_LAUNCHED(L);
   return CVCB_OK;
