@@ -282,6 +282,12 @@ struct HopArgs {
   SF rup;
   const double *alpha;
   DotFinish fin;
+  // FP64 sweeps that end in a residual (RES): the field it is taken from, the
+  // coefficients of A, whether the residual is stored, and where this sweep's
+  // partials of |residual|^2 start among the dot_np of a right-hand side
+  SF sub;
+  double ra, rb;
+  int store_res, dot_off;
 };
 
 // |a|^2 of one site, accumulated in FP64
@@ -329,7 +335,64 @@ struct HopMinBlocks {
   static constexpr int value = NR == 1 ? 3 : NR <= 3 ? 2 : 1;
 };
 
-template <class SF, class LF, int NR, bool G5IN, bool G5HOP, bool AUX>
+// RES (FP64, one rhs per thread): the sweep ends in a residual whose norm is
+// taken along, instead of passes of its own over the fields.
+//   1: sub - (D2 aux + D1 c hop), stored in out if store_res
+//   2: out = D1 (c hop) + D2 aux, and aux - A out + c hop, A = ra + i rb g5
+template <int RES, class SF, class LF>
+__device__ __forceinline__ double hop_epilogue(const HopArgs<SF, LF> &A, int r, int i,
+                                               const Spinor<typename SF::R> &h) {
+  using R = typename SF::R;  // h = c [g5] hop
+  Spinor<R> o = diag_op((R)A.d1a, (R)A.d1b, h);
+  const Spinor<R> aux = A.aux.load(r, i);
+  const Spinor<R> x = diag_op((R)A.d2a, (R)A.d2b, aux);
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o.c[s][q] = o.c[s][q] + x.c[s][q];
+  Spinor<R> res;
+  if (RES == 1) {
+    const Spinor<R> b = A.sub.load(r, i);
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) res.c[s][q] = b.c[s][q] - o.c[s][q];
+    if (A.store_res) A.out.store(r, i, res);
+  } else {
+    A.out.store(r, i, o);
+    const Spinor<R> ax = diag_op((R)A.ra, (R)A.rb, o);
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) res.c[s][q] = (aux.c[s][q] - ax.c[s][q]) + h.c[s][q];
+  }
+  double n2 = 0.0;
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      n2 = fma((double)res.c[s][q].re, (double)res.c[s][q].re, n2);
+      n2 = fma((double)res.c[s][q].im, (double)res.c[s][q].im, n2);
+    }
+  return n2;
+}
+// lanes of this thread's warp that exist (a block need not be whole warps)
+__device__ __forceinline__ unsigned warp_mask() {
+  const int t = threadIdx.y * blockDim.x + threadIdx.x, left = blockDim.x * blockDim.y - (t & ~31);
+  return left >= 32 ? 0xffffffffu : (1u << left) - 1;
+}
+// partials of a row of bx threads (one rhs; whole warps, or 16 lanes each)
+__host__ __device__ inline int res_parts(int bx) { return bx < 32 ? 1 : bx / 32; }
+template <class SF, class LF>
+__device__ __forceinline__ void store_res_part(const HopArgs<SF, LF> &A, int r, bool act, double n2,
+                                               int sb) {
+  const int w = blockDim.x < 32 ? blockDim.x : 32;
+  for (int o = w >> 1; o > 0; o >>= 1) n2 += __shfl_down_sync(warp_mask(), n2, o, w);
+  if (act && (threadIdx.x & (w - 1)) == 0)
+    A.dot_part[(size_t)r * A.dot_np + A.dot_off + sb * res_parts(blockDim.x) + threadIdx.x / w] = n2;
+}
+
+template <class SF, class LF, int NR, bool G5IN, bool G5HOP, bool AUX, int RES = 0>
 __device__ __forceinline__ void eo_hop_body(const HopArgs<SF, LF> &A) {
   using R = typename SF::R;
   const int r0 = (blockIdx.x * blockDim.y + threadIdx.y) * NR;
@@ -347,9 +410,16 @@ __device__ __forceinline__ void eo_hop_body(const HopArgs<SF, LF> &A) {
   const int qoff = (1 - p) * g.Vh;
   for (int sb = blockIdx.y; sb * (int)blockDim.x < g.Vh; sb += gridDim.y) {
     const int i = sb * blockDim.x + threadIdx.x;
-    if (i >= g.Vh) return;
-    const SiteCoord cd = site_coord(g, p, i);
-    const int self = p * g.Vh + i;
+    if (RES) {  // the whole warp takes part in the sum of the norm
+      if (__all_sync(warp_mask(), i >= g.Vh)) {
+        store_res_part(A, r0, true, 0.0, sb);
+        continue;
+      }
+    } else if (i >= g.Vh) {
+      return;
+    }
+    const SiteCoord cd = site_coord(g, p, RES && i >= g.Vh ? g.Vh - 1 : i);
+    const int self = p * g.Vh + cd.lex / 2;
 
     Spinor<R> acc[NR];
 #pragma unroll
@@ -394,6 +464,10 @@ __device__ __forceinline__ void eo_hop_body(const HopArgs<SF, LF> &A) {
       for (int s = 0; s < 4; ++s)
 #pragma unroll
         for (int q = 0; q < 3; ++q) o.c[s][q] = c * acc[k].c[s][q];
+      if constexpr (RES != 0) {
+        store_res_part(A, r0, true, i < g.Vh ? hop_epilogue<RES>(A, r0, i, o) : 0.0, sb);
+        continue;
+      }
       o = diag_op((R)A.d1a, (R)A.d1b, o);
       if (AUX) {
         const Spinor<R> x = diag_op((R)A.d2a, (R)A.d2b, A.aux.load(r0 + k, i));
@@ -413,9 +487,9 @@ __global__ void __launch_bounds__(kHopMaxThreads, HopMinBlocks<NR>::value)
   eo_hop_body<SF, LF, NR, G5IN, G5HOP, AUX>(A);
 }
 
-template <class LF, bool G5IN, bool G5HOP, bool AUX>
+template <class LF, bool G5IN, bool G5HOP, bool AUX, int RES = 0>
 __global__ void __launch_bounds__(kHopMaxThreads) k_eo_hop64(HopArgs<F64Acc, LF> A) {
-  eo_hop_body<F64Acc, LF, 1, G5IN, G5HOP, AUX>(A);
+  eo_hop_body<F64Acc, LF, 1, G5IN, G5HOP, AUX, RES>(A);
 }
 
 // ---- two right-hand sides per thread in packed FP32x2 arithmetic -----------
@@ -684,7 +758,7 @@ __host__ __device__ constexpr size_t staged_smem_bytes(int bx) {
   return (size_t)8 * 9 * bx * sizeof(Cx<R>) + (size_t)8 * bx * sizeof(int);
 }
 
-template <class SF, class LF, bool G5IN, bool G5HOP, bool AUX>
+template <class SF, class LF, bool G5IN, bool G5HOP, bool AUX, int RES = 0>
 __device__ __forceinline__ void eo_hop_staged_body(const HopArgs<SF, LF> &A) {
   using R = typename SF::R;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -713,6 +787,7 @@ __device__ __forceinline__ void eo_hop_staged_body(const HopArgs<SF, LF> &A) {
       }
     }
     __syncthreads();
+    double n2 = 0.0;
     if (valid && act) {
       Spinor<R> acc;
 #pragma unroll
@@ -742,16 +817,21 @@ __device__ __forceinline__ void eo_hop_staged_body(const HopArgs<SF, LF> &A) {
       for (int s = 0; s < 4; ++s)
 #pragma unroll
         for (int q = 0; q < 3; ++q) o.c[s][q] = c * acc.c[s][q];
-      o = diag_op((R)A.d1a, (R)A.d1b, o);
-      if (AUX) {
-        const Spinor<R> x = diag_op((R)A.d2a, (R)A.d2b, A.aux.load(r, i));
+      if constexpr (RES != 0) {
+        n2 = hop_epilogue<RES>(A, r, i, o);
+      } else {
+        o = diag_op((R)A.d1a, (R)A.d1b, o);
+        if (AUX) {
+          const Spinor<R> x = diag_op((R)A.d2a, (R)A.d2b, A.aux.load(r, i));
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
+          for (int s = 0; s < 4; ++s)
 #pragma unroll
-          for (int q = 0; q < 3; ++q) o.c[s][q] = o.c[s][q] + x.c[s][q];
+            for (int q = 0; q < 3; ++q) o.c[s][q] = o.c[s][q] + x.c[s][q];
+        }
+        A.out.store(r, i, o);
       }
-      A.out.store(r, i, o);
     }
+    if (RES) store_res_part(A, r, act, n2, sb);
     __syncthreads();  // the next site block overwrites the staged links
   }
 }
@@ -764,9 +844,9 @@ template <class SF, class LF, bool G5IN, bool G5HOP, bool AUX>
 __global__ void __launch_bounds__(kHopMaxThreads, 2) k_eo_hop_staged(HopArgs<SF, LF> A) {
   eo_hop_staged_body<SF, LF, G5IN, G5HOP, AUX>(A);
 }
-template <class LF, bool G5IN, bool G5HOP, bool AUX>
+template <class LF, bool G5IN, bool G5HOP, bool AUX, int RES = 0>
 __global__ void __launch_bounds__(128, 4) k_eo_hop_staged64(HopArgs<F64Acc, LF> A) {
-  eo_hop_staged_body<F64Acc, LF, G5IN, G5HOP, AUX>(A);
+  eo_hop_staged_body<F64Acc, LF, G5IN, G5HOP, AUX, RES>(A);
 }
 
 }  // namespace cvcb

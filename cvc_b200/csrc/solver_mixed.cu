@@ -286,9 +286,9 @@ __device__ __forceinline__ PairLanes pair_lanes(int pr, int nrhs, const int *ski
 __device__ __forceinline__ float lane_re(const CP &c, int l) { return l ? c.re.y : c.re.x; }
 __device__ __forceinline__ float lane_im(const CP &c, int l) { return l ? c.im.y : c.im.x; }
 
-// x64 += x_s / scale; x_s = 0
-__global__ void k_absorb_pt(F64Acc x64, P32 xs, const double *scale, const int *skip, int nsites,
-                            int nrhs) {
+// x64 += x_s / scale (x64 = x_s / scale the first time: `fresh`); x_s = 0
+__global__ void k_absorb_pt(F64Acc x64, P32 xs, const double *scale, const int *skip,
+                            const int *fresh, int nsites, int nrhs) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int pr = blockIdx.y;
   const PairLanes m = pair_lanes(pr, nrhs, skip);
@@ -299,7 +299,13 @@ __global__ void k_absorb_pt(F64Acc x64, P32 xs, const double *scale, const int *
     if (!(l ? m.act_b : m.act_a)) continue;
     const int r = m.ra + l;
     const double w = 1.0 / scale[r];
-    Spinor<double> xv = x64.load(r, s);
+    Spinor<double> xv;
+    if (fresh[r]) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) xv.c[k / 3][k % 3] = cx(0.0, 0.0);
+    } else {
+      xv = x64.load(r, s);
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k)
 #pragma unroll
@@ -471,16 +477,23 @@ __global__ void __launch_bounds__(kRedThreads)
   }
 }
 
-// Reliable update, step 1: x64 += x_s / scale; x_s = 0 (rhs with skip[r] == 0)
+// Reliable update, step 1: x64 += x_s / scale (the first time x64 = x_s /
+// scale); x_s = 0 (rhs with skip[r] == 0)
 template <class XF>
-__global__ void k_absorb(F64Acc x64, XF xs, const double *scale, const int *skip, int nsites,
-                         int nrhs) {
+__global__ void k_absorb(F64Acc x64, XF xs, const double *scale, const int *skip, const int *fresh,
+                         int nsites, int nrhs) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y;
   if (s >= nsites || r >= nrhs || skip[r]) return;
   using RX = typename XF::R;
   const double w = 1.0 / scale[r];
-  Spinor<double> xv = x64.load(r, s);
+  Spinor<double> xv;
+  if (fresh[r]) {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) xv.c[k / 3][k % 3] = cx(0.0, 0.0);
+  } else {
+    xv = x64.load(r, s);
+  }
   const Spinor<RX> d = xs.load(r, s);
   Spinor<RX> z;
 #pragma unroll
@@ -495,20 +508,6 @@ __global__ void k_absorb(F64Acc x64, XF xs, const double *scale, const int *skip
   xs.store(r, s, z);
 }
 
-// r_hat = b_hat - y; returns |r_hat|^2
-struct RedRhat {
-  F64Acc bhat, y;
-  __device__ double operator()(int r, int s) const {
-    const Spinor<double> b = bhat.load(r, s);
-    Spinor<double> v = y.load(r, s);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) v.c[k][c] = b.c[k][c] - v.c[k][c];
-    y.store(r, s, v);
-    return norm2(v);
-  }
-};
 struct EpiStore {
   double *dst;
   __device__ void operator()(int r, double t) const { dst[r] = t; }
@@ -633,36 +632,65 @@ __global__ void k_copy(SF dst, SF src, const int *skip, int nsites, int nrhs) {
   dst.store(r, s, src.load(r, s));
 }
 
-// t = D v (site-diagonal), FP64 fields
-__global__ void k_diag64(F64Acc out, F64Acc in, double a, double b, int nsites, int nrhs) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y;
-  if (s >= nsites || r >= nrhs) return;
-  out.store(r, s, diag_op(a, b, in.load(r, s)));
-}
-
-// |v|^2 over the full lattice (both halves), FP64
+// |v|^2, FP64
 struct RedNorm64 {
   F64Acc v;
   __device__ double operator()(int r, int s) const { return norm2(v.load(r, s)); }
 };
 
-// y = a - b on full fields
-struct RedResid {
-  F64Acc a, b;
-  __device__ double operator()(int r, int s) const {
-    const Spinor<double> u = a.load(r, s), v = b.load(r, s);
-    double t = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const double dr = u.c[k][c].re - v.c[k][c].re, di = u.c[k][c].im - v.c[k][c].im;
-        t += dr * dr + di * di;
-      }
-    return t;
-  }
+// Sources of a batch from CVC layout to the device layout, with what the start
+// needs of them in the same pass: t = D b on the even sites (D = A^-1: the
+// input of the hop that forms b_hat) and per-block partials of |b|^2.
+// blockIdx.y = rhs; tiles as in k_spinor_aos_to_eo.
+struct FieldPtrs {
+  double2 *p[kMaxBatch];
 };
+constexpr int kIoTile = 64, kIoThreads = 128;
+__global__ void __launch_bounds__(kIoThreads)
+    k_sources_in(double2 *__restrict__ b, double2 *__restrict__ t, const __grid_constant__ FieldPtrs src,
+                 Geom g, double da, double db, double *__restrict__ part, int np) {
+  __shared__ double2 tile[kIoTile * 13];
+  __shared__ double sw[kIoThreads / 32];
+  const int r = blockIdx.y, base = blockIdx.x * kIoTile, n = min(kIoTile, g.V - base);
+  const double2 *f = src.p[r] + (size_t)base * 12;
+  double n2 = 0.0;
+  for (int q = threadIdx.x; q < n * 12; q += kIoThreads) {
+    const double2 v = __ldg(f + q);
+    n2 = fma(v.x, v.x, fma(v.y, v.y, n2));
+    tile[q + q / 12] = v;
+  }
+  __syncthreads();
+  const size_t fs = (size_t)12 * g.V;
+  for (int q = threadIdx.x; q < kIoTile * 12; q += kIoThreads) {
+    const int k = q / kIoTile, s = q % kIoTile;
+    if (s >= n) continue;
+    const int j = lex_to_eo(g, base + s);
+    const double2 v = tile[s * 13 + k];
+    b[r * fs + (size_t)k * g.V + j] = v;
+    const double bb = k < 6 ? db : -db;
+    if (j < g.Vh) t[r * fs + (size_t)k * g.V + j] = make_double2(da * v.x - bb * v.y, da * v.y + bb * v.x);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) n2 += __shfl_down_sync(0xffffffffu, n2, o);
+  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = n2;
+  __syncthreads();
+  if (threadIdx.x == 0) part[(size_t)r * np + blockIdx.x] = (sw[0] + sw[1]) + (sw[2] + sw[3]);
+}
+
+// Solutions of a batch back to CVC layout.
+__global__ void __launch_bounds__(kIoThreads)
+    k_solutions_out(const __grid_constant__ FieldPtrs dst, const double2 *__restrict__ x, Geom g) {
+  __shared__ double2 tile[kIoTile * 13];
+  const int r = blockIdx.y, base = blockIdx.x * kIoTile, n = min(kIoTile, g.V - base);
+  const size_t fs = (size_t)12 * g.V;
+  for (int q = threadIdx.x; q < kIoTile * 12; q += kIoThreads) {
+    const int k = q / kIoTile, s = q % kIoTile;
+    if (s < n) tile[s * 13 + k] = __ldg(x + r * fs + (size_t)k * g.V + lex_to_eo(g, base + s));
+  }
+  __syncthreads();
+  double2 *f = dst.p[r] + (size_t)base * 12;
+  for (int q = threadIdx.x; q < n * 12; q += kIoThreads) f[q] = tile[q + q / 12];
+}
 
 }  // namespace
 
@@ -773,6 +801,7 @@ struct Batch {
   int dot_np = 0;
   int *ru_skip;   // per rhs: 1 = skip in the reliable update
   int *rst_skip;  // per rhs: 0 = restart the direction from the residual
+  int *fresh;     // per rhs: 1 = x64 holds nothing yet
   BatchRed br;
   LF links;
   L64 links64;
@@ -1029,6 +1058,54 @@ struct Batch {
     }
   }
 
+  // FP64 sweep that ends in a residual (RES, eo_hop_body): partials of its
+  // norm at dot_part[rhs * np + off ...]; res_np() of them per rhs and sweep
+  LaunchShape shape_f64() const {
+    LaunchShape sh = sizeof(typename SF::R) != 8 ? shape64 : shape;
+    if (sh.bx != 16 && sh.bx % 32) sh = LaunchShape{};  // the sums want whole (half) warps per row
+    sh.by = std::min(sh.by, n);
+    return sh;
+  }
+  int res_np() const {
+    const LaunchShape sh = shape_f64();
+    return (g.Vh + sh.bx - 1) / sh.bx * res_parts(sh.bx);
+  }
+  template <int RES>
+  int hop64_res(HopArgs<F64Acc, L64> a, int np, int off) {
+    const LaunchShape sh = shape_f64();
+    a.dot_part = dot_part;
+    a.dot_np = np;
+    a.dot_off = off;
+    const int site_blocks = (g.Vh + sh.bx - 1) / sh.bx;
+    dim3 block(sh.bx, sh.by), grid((n + sh.by - 1) / sh.by, std::min(site_blocks, 65535));
+    if (sh.by > 1) {
+      auto kern = k_eo_hop_staged64<L64, false, false, true, RES>;
+      const size_t smem = staged_smem_bytes<double>(sh.bx);
+      CVCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxStagedSmem));
+      kern<<<grid, block, smem, L->stream>>>(a);
+    } else {
+      k_eo_hop64<L64, false, false, true, RES><<<grid, block, 0, L->stream>>>(a);
+    }
+    CVCB_LAUNCHED(L);
+    return CVCB_OK;
+  }
+  // r_hat = b_hat - M(mu) x64 into y64, and |r_hat|^2 with the new unit
+  int residual64(const int *skip) {
+    double ia, ib;
+    ainv(mu, ia, ib);
+    CVCB_TRY((hop<F64Acc, L64, false, false, false>(f64(t64, 0), f64(x64, 1), f64(x64, 1), links64, 0,
+                                                    skip, ia, ib, 0, 0, -0.5)));
+    HopArgs<F64Acc, L64> a{f64(y64, 1), f64(t64, 0), f64(x64, 1), links64, EoGeom{g, 1}, n, skip,
+                           1, 0, ka(), mu, 0.5};
+    a.sub = f64(bh64, 1);
+    a.store_res = 1;
+    const int np = res_np();
+    CVCB_TRY(hop64_res<1>(a, np, 0));
+    k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(dot_part, np, EpiRhat{S}, skip);
+    CVCB_LAUNCHED(L);
+    return CVCB_OK;
+  }
+
   // FP64: out_o = M(m) in_o  (t64 even half as intermediate)
   int schur64(double2 *out, double2 *in, double m, const int *skip) {
     double ia, ib;
@@ -1053,26 +1130,25 @@ struct Batch {
   // absorb = false is the start from x = 0, where M x = 0 needs no sweep.
   int reliable_update(bool absorb) {
     dim3 eg((g.Vh + 127) / 128, n);
+    dim3 rg(red_blocks_sites(g.Vh), n);
+    const F64Acc rhat = f64(absorb ? y64 : bh64, 1);
     if (absorb) {
       if constexpr (std::is_same<XF, P32>::value)
         k_absorb_pt<<<dim3(eg.x, (n + 1) / 2), 128, 0, L->stream>>>(f64(x64, 1), xs, S.scale,
-                                                                    ru_skip, g.Vh, n);
+                                                                    ru_skip, fresh, g.Vh, n);
       else
-        k_absorb<<<eg, 128, 0, L->stream>>>(f64(x64, 1), xs, S.scale, ru_skip, g.Vh, n);
+        k_absorb<<<eg, 128, 0, L->stream>>>(f64(x64, 1), xs, S.scale, ru_skip, fresh, g.Vh, n);
       CVCB_LAUNCHED(L);
-      CVCB_TRY(schur64(y64, x64, mu, ru_skip));
+      CVCB_TRY(residual64(ru_skip));
     } else {
-      CVCB_CUDA(cudaMemsetAsync(y64, 0, (size_t)12 * g.V * sizeof(double2) * n, L->stream));
+      k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedNorm64{rhat}, EpiRhat{S}, g.Vh, br, ru_skip);
+      CVCB_LAUNCHED(L);
     }
-    dim3 rg(red_blocks_sites(g.Vh), n);
-    k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedRhat{f64(bh64, 1), f64(y64, 1)},
-                                                    EpiRhat{S}, g.Vh, br, ru_skip);
-    CVCB_LAUNCHED(L);
     if constexpr (kPairTiled<SF>)
-      k_to_sloppy_pt<<<dim3(eg.x, (n + 1) / 2), 128, 0, L->stream>>>(yo, f64(y64, 1), S.scale,
-                                                                      ru_skip, g.Vh, n);
+      k_to_sloppy_pt<<<dim3(eg.x, (n + 1) / 2), 128, 0, L->stream>>>(yo, rhat, S.scale, ru_skip,
+                                                                      g.Vh, n);
     else
-      k_to_sloppy<<<eg, 128, 0, L->stream>>>(yo, f64(y64, 1), S.scale, ru_skip, g.Vh, n);
+      k_to_sloppy<<<eg, 128, 0, L->stream>>>(yo, rhat, S.scale, ru_skip, g.Vh, n);
     CVCB_LAUNCHED(L);
     CVCB_TRY(dag_sloppy(rs, yo, ru_skip));
     k_reduce_rhs<<<rg, kRedThreads, 0, L->stream>>>(RedNormS<SF>{rs}, EpiRR{S}, g.Vh, br, ru_skip);
@@ -1195,10 +1271,11 @@ int setup_batch(cvcb_lattice *L, Batch<SF, XF, LF> &B, int n, bool with_fp64 = t
   const size_t xsl = sloppy_field_bytes<XF>(g.Vh, n);
   const size_t nrm = sloppy_scale_bytes<SF>(g.Vh, n);
   auto rnd = [](size_t b) { return (b + 255) & ~size_t(255); };  // every piece 256-aligned
-  const size_t scal = 8 * rnd(sizeof(double) * kMaxBatch) + 3 * rnd(sizeof(int) * kMaxBatch);
+  const size_t scal = 8 * rnd(sizeof(double) * kMaxBatch) + 4 * rnd(sizeof(int) * kMaxBatch);
   const size_t part = rnd(sizeof(double) * kMaxRedBlocks * kMaxBatch * 2) +
                       rnd(sizeof(unsigned) * kMaxBatch);
-  const size_t dotb = sizeof(double) * (size_t)n * (g.Vh / 32 + 64);
+  // partial sums: at most one per 16 sites of both parities
+  const size_t dotb = sizeof(double) * (size_t)n * (g.V / 16 + 512);
   const size_t total = 5 * rnd(f64) + 6 * (rnd(sl) + rnd(nrm)) + rnd(xsl) + scal + part +
                        rnd(dotb);
   void *mem;
@@ -1237,6 +1314,7 @@ int setup_batch(cvcb_lattice *L, Batch<SF, XF, LF> &B, int n, bool with_fp64 = t
   B.S.done = (int *)take(sizeof(int) * kMaxBatch);
   B.ru_skip = (int *)take(sizeof(int) * kMaxBatch);
   B.rst_skip = (int *)take(sizeof(int) * kMaxBatch);
+  B.fresh = (int *)take(sizeof(int) * kMaxBatch);
   B.br.partials = (double *)take(sizeof(double) * kMaxRedBlocks * kMaxBatch * 2);
   B.br.counters = (unsigned *)take(sizeof(unsigned) * kMaxBatch);
   B.dot_part = (double *)take(dotb);
@@ -1392,32 +1470,41 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
   const Geom &g = L->g;
   const size_t fs = (size_t)12 * g.V;
   dim3 eg((g.Vh + 127) / 128, n);
-  dim3 egf((g.V + 127) / 128, n);
-  dim3 rg(red_blocks_sites(g.Vh), n), rgf(red_blocks_sites(g.V), n);
+  dim3 rg(red_blocks_sites(g.Vh), n);
 
-  for (int i = 0; i < n; ++i) CVCB_TRY(spinor_in(L, B.b64 + i * fs, b[i], g.V));
-  if (inputs_read) CVCB_CUDA(cudaEventRecord(inputs_read, L->stream));
   CVCB_TRY(tune_shape(L, B, P->precision, P->link_recon, P->block_threads));
   if (sizeof(typename SF::R) != 8) CVCB_TRY(tune_shape64(L, B));
   if (shape_out) *shape_out = B.shape;
 
+  // sources in: host fields through y64 (not in use yet) as they are
+  FieldPtrs io;
+  for (int i = 0; i < n; ++i) {
+    io.p[i] = reinterpret_cast<double2 *>(const_cast<double *>(b[i]));
+    if (!is_device_ptr(b[i])) {
+      io.p[i] = B.y64 + i * fs;
+      CVCB_CUDA(cudaMemcpyAsync(io.p[i], b[i], fs * sizeof(double2), cudaMemcpyHostToDevice, L->stream));
+    }
+  }
+  const dim3 iog((g.V + kIoTile - 1) / kIoTile, n);
+  double ia, ib;
+  B.ainv(B.mu, ia, ib);
+  k_sources_in<<<iog, kIoThreads, 0, L->stream>>>(B.b64, B.t64, io, g, ia, ib, B.dot_part, iog.x);
+  CVCB_LAUNCHED(L);
   // |b|^2 over the full lattice
   double *bnorm2 = B.S.rn2;  // temporary use
-  k_reduce_rhs<<<rgf, kRedThreads, 0, L->stream>>>(RedNorm64{B.f64full(B.b64)},
-                                                   EpiStore{bnorm2}, g.V, B.br, nullptr);
+  k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(B.dot_part, iog.x, EpiStore{bnorm2}, (const int *)nullptr);
   CVCB_LAUNCHED(L);
+  if (inputs_read) CVCB_CUDA(cudaEventRecord(inputs_read, L->stream));
   std::vector<double> hb2(n);
   CVCB_TRY(fetch(L, bnorm2, n, 0));
   // b_hat = b_o + 1/2 H_oe A_ee^-1 b_e
-  double ia, ib;
-  B.ainv(B.mu, ia, ib);
-  k_diag64<<<eg, 128, 0, L->stream>>>(B.f64(B.t64, 0), B.f64(B.b64, 0), ia, ib, g.Vh, n);
-  CVCB_LAUNCHED(L);
   CVCB_TRY((B.template hop<F64Acc, L64, false, false, true>(B.f64(B.bh64, 1), B.f64(B.t64, 0),
                                                             B.f64(B.b64, 1), B.links64, 1,
                                                             nullptr, 1, 0, 1, 0, 0.5)));
-  // x = 0, x_s = 0; reliable update from x = 0 gives r_hat = b_hat, r_N = b_N
-  CVCB_CUDA(cudaMemsetAsync(B.x64, 0, fs * n * sizeof(double2), L->stream));
+  // x = 0 (x64 is written by the first absorb), x_s = 0; reliable update from
+  // x = 0 gives r_hat = b_hat, r_N = b_N
+  std::vector<int> fresh(n, 1);
+  CVCB_TRY(put_flags(L, B.fresh, fresh, n));
   CVCB_TRY(B.reliable_update(false));
   // x_s = 0 (all-zero bits are 0.0), p = r_s
   CVCB_CUDA(cudaMemsetAsync(B.xs_mem, 0, B.xs_bytes, L->stream));
@@ -1584,6 +1671,10 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
       k_dir_strip<<<eg, 128, 0, L->stream>>>(B.p, B.rs, B.ru_skip, g.Vh, n);
     CVCB_LAUNCHED(L);
     CVCB_TRY(B.reliable_update(true));
+    bool first = false;  // first absorb of some right-hand side
+    for (int i = 0; i < n; ++i)
+      if (!skip[i] && fresh[i]) fresh[i] = 0, first = true;
+    if (first) CVCB_TRY(put_flags(L, B.fresh, fresh, n));
     if constexpr (kPairTiled<SF>) {
       k_cdot_pt<<<dim3(rg.x, (n + 1) / 2), kRedThreads, 0, L->stream>>>(
           B.rs, B.p, g.Vh, n, B.br.partials, B.br.counters, B.ru_skip, B.S.pAp, B.S.alpha);
@@ -1639,23 +1730,44 @@ int run_batch(cvcb_lattice *L, double *const *x, const double *const *b, int n,
   B.recs.clear();
   if (rc != CVCB_OK) return rc;
 
-  // x_e = A^-1 (b_e + 1/2 H_eo x_o)
-  CVCB_TRY((B.template hop<F64Acc, L64, false, false, true>(B.f64(B.x64, 0), B.f64(B.x64, 1),
-                                                            B.f64(B.b64, 0), B.links64, 0,
-                                                            nullptr, ia, ib, ia, ib, 0.5)));
-  // final FP64 check |b - Q x| / |b| over the whole lattice: t_p = (Q x)_p =
-  // A x_p - 1/2 H_pq x_q for both parities, batched over the rhs
+  // right-hand sides that never absorbed (zero, or met the target at once): x_o = 0
+  for (int i = 0; i < n; ++i)
+    if (fresh[i])
+      CVCB_CUDA(cudaMemset2DAsync(B.x64 + i * fs + g.Vh, (size_t)g.V * sizeof(double2), 0,
+                                  (size_t)g.Vh * sizeof(double2), 12, L->stream));
+  // x_e = A^-1 (b_e + 1/2 H_eo x_o), and the final FP64 check |b - Q x| / |b|
+  // over the whole lattice, Q x = A x_p - 1/2 H_pq x_q: the even rows from the
+  // hop that x_e is made of, the odd rows with a sweep of their own
   double worst = 0.0;
   int nconv = 0;
-  for (int par = 0; par < 2; ++par)
-    CVCB_TRY((B.template hop<F64Acc, L64, false, false, true>(
-        B.f64(B.t64, par), B.f64(B.x64, 1 - par), B.f64(B.x64, par), B.links64, par, nullptr, 1.0,
-        0.0, B.ka(), B.mu, -0.5)));
-  k_reduce_rhs<<<rgf, kRedThreads, 0, L->stream>>>(
-      RedResid{B.f64full(B.t64), B.f64full(B.b64)}, EpiStore{B.S.rhat2}, g.V, B.br, nullptr);
-  CVCB_LAUNCHED(L);
+  {
+    const int np = B.res_np();
+    HopArgs<F64Acc, L64> e{B.f64(B.x64, 0), B.f64(B.x64, 1), B.f64(B.b64, 0), B.links64, EoGeom{g, 0},
+                           n, nullptr, ia, ib, ia, ib, 0.5};
+    e.ra = B.ka();
+    e.rb = B.mu;
+    CVCB_TRY(B.template hop64_res<2>(e, 2 * np, 0));
+    HopArgs<F64Acc, L64> o{B.f64(B.t64, 1), B.f64(B.x64, 0), B.f64(B.x64, 1), B.links64, EoGeom{g, 1},
+                           n, nullptr, 1.0, 0.0, B.ka(), B.mu, -0.5};
+    o.sub = B.f64(B.b64, 1);
+    CVCB_TRY(B.template hop64_res<1>(o, 2 * np, np));
+    k_dot_finish<<<n, kRedThreads, 0, L->stream>>>(B.dot_part, 2 * np, EpiStore{B.S.rhat2},
+                                                   (const int *)nullptr);
+    CVCB_LAUNCHED(L);
+  }
   CVCB_TRY(fetch(L, B.S.rhat2, n, 2));
-  for (int i = 0; i < n; ++i) CVCB_TRY(spinor_out(L, x[i], B.x64 + i * fs, g.V));
+  // solutions out: one launch for the fields in device memory
+  int ndev = 0;
+  for (int i = 0; i < n; ++i) {
+    io.p[i] = reinterpret_cast<double2 *>(x[i]);
+    ndev += is_device_ptr(x[i]);
+  }
+  if (ndev == n) {
+    k_solutions_out<<<iog, kIoThreads, 0, L->stream>>>(io, B.x64, g);
+    CVCB_LAUNCHED(L);
+  } else {
+    for (int i = 0; i < n; ++i) CVCB_TRY(spinor_out(L, x[i], B.x64 + i * fs, g.V));
+  }
   CVCB_CUDA(cudaStreamSynchronize(L->stream));
   mailbox(L, 2, rhat2, n);
   for (int i = 0; i < n; ++i) {
