@@ -209,10 +209,11 @@ int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, d
 // layout, which cost two field passes more than the operator itself.  Thread =
 // lexicographic site; a spinor is six 32-byte loads (one whole sector each; V4)
 // or twelve 16-byte ones (fields off a 32-byte boundary).  Same terms in the
-// same order as k_tm_full_f64: the same bits.  A call takes 17 us at 4^3 x 8
-// (25 with the two copies), 29 (44) at 22 x 14 x 10 x 18 and 613 (818) at
-// 32^3 x 64; compulsory traffic there 2.0 GB, 0.31 ms.  Bound by L1: the
-// strided spinor loads keep its data pipe 82 % busy.
+// same order as k_tm_full_f64: the same bits.  A call takes 29 us at
+// 22 x 14 x 10 x 18 (44 with the two copies) and 613 (818) at 32^3 x 64;
+// compulsory traffic there 2.0 GB, 0.31 ms.  Bound by L1: the strided spinor
+// loads keep its data pipe 82 % busy, and so does a copy through shared memory
+// by cp.async (644 us).
 template <bool V4>
 __device__ __forceinline__ Spinor<double> load_spinor_cvc(const double2 *__restrict__ f, int lex) {
   const double2 *q = f + (size_t)lex * 12;
@@ -308,6 +309,108 @@ __global__ void __launch_bounds__(kCvcThreads, 3)
   store_spinor_cvc<V4>(out, lex, r);
 }
 
+// The same for small lattices, where the GPU waits for one site's directions one
+// after the other: block = 32 lexicographic sites, warp d = direction (t-, t+,
+// x-, ...), every warp loads one neighbour and leaves its transported half
+// spinor in shared memory, warps 0..2 sum the sink colours 0..2 in the order
+// of the kernels above (the same bits) and add the diagonal.
+constexpr int kCvcSplitThreads = 256;
+// Up to here: 14.2 against 16.7 us a call at 512 sites, 15.5 against 17.5 at
+// 8192; at 12,000 18.8 against 18.2, at 55,440 32.6 against 27.
+constexpr int kCvcSplitSites = 8192;
+
+template <int MU, bool DAG, bool V4>
+__device__ __forceinline__ void cvc_split_dir(double2 (*sh)[32], const double2 *__restrict__ in,
+                                              const double2 *__restrict__ U, const Geom &g,
+                                              const SiteCoord &cd, int self, int qoff, int lane) {
+  const int j = nb_lex(g, cd, MU, DAG ? -1 : +1);
+  const Link<double> W = load_link64(U, g.V, MU, DAG ? qoff + (j >> 1) : self);
+  const HalfSpinor<double> h = project(MU, DAG ? +1 : -1, load_spinor_cvc<V4>(in, j));
+  const HalfSpinor<double> u = DAG ? link_dag_mul(W, h) : link_mul(W, h);
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh[3 * b + c][lane] = make_double2(u.c[b][c].re, u.c[b][c].im);
+}
+
+// one colour of accum_recon: acc[spin] += (1 + S g_mu)-reconstruction of (u0, u1)
+template <int MU, int S>
+__device__ __forceinline__ void cvc_recon(Cx<double> (&acc)[4], double2 a, double2 b) {
+  const Cx<double> u0 = cx(a.x, a.y), u1 = cx(b.x, b.y);
+  acc[0] = acc[0] + u0;
+  acc[1] = acc[1] + u1;
+  if (MU == 0) {
+    acc[2] = acc[2] + sgn(-S, u0);
+    acc[3] = acc[3] + sgn(-S, u1);
+  } else if (MU == 1) {
+    acc[2] = acc[2] + sgn(S, mul_i(u1));
+    acc[3] = acc[3] + sgn(S, mul_i(u0));
+  } else if (MU == 2) {
+    acc[2] = acc[2] + sgn(S, u1);
+    acc[3] = acc[3] + sgn(-S, u0);
+  } else {
+    acc[2] = acc[2] + sgn(S, mul_i(u0));
+    acc[3] = acc[3] + sgn(-S, mul_i(u1));
+  }
+}
+
+template <bool G5OUT, bool V4>
+__global__ void __launch_bounds__(kCvcSplitThreads)
+    k_tm_full_cvc_split(double2 *__restrict__ out, const double2 *__restrict__ in,
+                        const double2 *__restrict__ U, Geom g, double a, double b, double c) {
+  __shared__ double2 sh[8][6][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lex = blockIdx.x * 32 + lane;
+  const bool valid = lex < g.V;
+  double2 f[4];  // the site's own spinor, one colour
+  if (valid && warp < 3)
+#pragma unroll
+    for (int sp = 0; sp < 4; ++sp) f[sp] = __ldg(in + (size_t)lex * 12 + 3 * sp + warp);
+  if (valid) {
+    SiteCoord cd;
+    const unsigned r0 = fdiv((unsigned)lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
+    cd.lex = lex;
+    cd.z = lex - (int)r0 * g.LZ;
+    cd.y = (int)(r0 - r1 * g.LY);
+    cd.x = (int)(r1 - r2 * g.LX);
+    cd.t = (int)r2;
+    const int par = (cd.t + cd.x + cd.y + cd.z) & 1;
+    const int self = par * g.Vh + (lex >> 1), qoff = (1 - par) * g.Vh;
+    switch (warp) {
+      case 0: cvc_split_dir<0, true, V4>(sh[0], in, U, g, cd, self, qoff, lane); break;
+      case 1: cvc_split_dir<0, false, V4>(sh[1], in, U, g, cd, self, qoff, lane); break;
+      case 2: cvc_split_dir<1, true, V4>(sh[2], in, U, g, cd, self, qoff, lane); break;
+      case 3: cvc_split_dir<1, false, V4>(sh[3], in, U, g, cd, self, qoff, lane); break;
+      case 4: cvc_split_dir<2, true, V4>(sh[4], in, U, g, cd, self, qoff, lane); break;
+      case 5: cvc_split_dir<2, false, V4>(sh[5], in, U, g, cd, self, qoff, lane); break;
+      case 6: cvc_split_dir<3, true, V4>(sh[6], in, U, g, cd, self, qoff, lane); break;
+      default: cvc_split_dir<3, false, V4>(sh[7], in, U, g, cd, self, qoff, lane); break;
+    }
+  }
+  __syncthreads();
+  if (!valid || warp >= 3) return;
+  Cx<double> acc[4];
+#pragma unroll
+  for (int sp = 0; sp < 4; ++sp) acc[sp] = cx(0.0, 0.0);
+  cvc_recon<0, +1>(acc, sh[0][warp][lane], sh[0][3 + warp][lane]);
+  cvc_recon<0, -1>(acc, sh[1][warp][lane], sh[1][3 + warp][lane]);
+  cvc_recon<1, +1>(acc, sh[2][warp][lane], sh[2][3 + warp][lane]);
+  cvc_recon<1, -1>(acc, sh[3][warp][lane], sh[3][3 + warp][lane]);
+  cvc_recon<2, +1>(acc, sh[4][warp][lane], sh[4][3 + warp][lane]);
+  cvc_recon<2, -1>(acc, sh[5][warp][lane], sh[5][3 + warp][lane]);
+  cvc_recon<3, +1>(acc, sh[6][warp][lane], sh[6][3 + warp][lane]);
+  cvc_recon<3, -1>(acc, sh[7][warp][lane], sh[7][3 + warp][lane]);
+#pragma unroll
+  for (int sp = 0; sp < 4; ++sp) {
+    const double bs = sp < 2 ? b : -b;  // i b g5
+    double2 o;
+    o.x = fma(c, acc[sp].re, fma(a, f[sp].x, -bs * f[sp].y));
+    o.y = fma(c, acc[sp].im, fma(a, f[sp].y, bs * f[sp].x));
+    if (G5OUT && sp >= 2) o = make_double2(-o.x, -o.y);
+    out[(size_t)lex * 12 + 3 * sp + warp] = o;
+  }
+}
+
 int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a, double b, double c,
                        bool g5out) {
   const Geom &g = L->g;
@@ -315,14 +418,15 @@ int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a,
   double2 *o = reinterpret_cast<double2 *>(out);
   const double2 *i = reinterpret_cast<const double2 *>(in);
   const bool v4 = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(in)) & 31) == 0;
-  if (g5out && v4)
-    k_tm_full_cvc<true, true><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
-  else if (g5out)
-    k_tm_full_cvc<true, false><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
-  else if (v4)
-    k_tm_full_cvc<false, true><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
-  else
-    k_tm_full_cvc<false, false><<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+  if (g.V <= kCvcSplitSites) {
+    auto kern = g5out ? (v4 ? k_tm_full_cvc_split<true, true> : k_tm_full_cvc_split<true, false>)
+                      : (v4 ? k_tm_full_cvc_split<false, true> : k_tm_full_cvc_split<false, false>);
+    kern<<<(g.V + 31) / 32, kCvcSplitThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+  } else {
+    auto kern = g5out ? (v4 ? k_tm_full_cvc<true, true> : k_tm_full_cvc<true, false>)
+                      : (v4 ? k_tm_full_cvc<false, true> : k_tm_full_cvc<false, false>);
+    kern<<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+  }
   CVCB_LAUNCHED(L);
   return CVCB_OK;
 }
