@@ -294,6 +294,14 @@ __global__ void k_grad_to_cvc(double *out, const double2 *G, Geom g) {
     }
 }
 
+// the gradient of the four source links, added at the source site
+struct SourceGrad {
+  double v[72];
+};
+__global__ void k_add_source_grad(double *out, const __grid_constant__ SourceGrad s) {
+  if (threadIdx.x < 72) out[threadIdx.x] += s.v[threadIdx.x];
+}
+
 double2 host_sum_partials(const std::vector<double2> &p, int pr, int nb) {
   double re = 0, im = 0;
   for (int b = 0; b < nb; ++b) {
@@ -371,8 +379,7 @@ static int columns(cvcb_lattice *L, double2 **props_out) {
     const int rc = solve_columns(L, static_cast<double *>(cvc), static_cast<double *>(bsrc),
                                  &S.params, L->mu, -L->mu, 60, 60, fstride);
     if (rc < 0) return rc;
-    for (int f = 0; f < 120; ++f)
-      CVCB_TRY(spinor_in(L, P + f * fs, static_cast<double *>(cvc) + f * fstride, g.V));
+    CVCB_TRY(spinors_in(L, P, static_cast<double *>(cvc), 120, false));
     S.have_props = true;
   }
   *props_out = P;
@@ -429,7 +436,7 @@ int pi_tangent(cvcb_lattice *L, int param, double *dconn) {
     return CVCB_ERR_ARG;
   }
   const Geom &g = L->g;
-  const size_t fs = (size_t)12 * g.V, fstride = (size_t)24 * g.V;
+  const size_t fstride = (size_t)24 * g.V;
   double2 *props;
   CVCB_TRY(columns(L, &props));
   void *cvc, *bsrc, *work;
@@ -439,7 +446,7 @@ int pi_tangent(cvcb_lattice *L, int param, double *dconn) {
   double *C = static_cast<double *>(cvc), *B = static_cast<double *>(bsrc),
          *W = static_cast<double *>(work);
   // columns back in CVC layout (C), right-hand sides of the tangent solves (B)
-  for (int f = 0; f < 120; ++f) CVCB_TRY(spinor_out(L, C + f * fstride, props + f * fs, g.V));
+  CVCB_TRY(spinors_out(L, C, props, 120, false));
   const double k2 = 1.0 / (2.0 * L->kappa * L->kappa);
   const int nb = (int)((fstride / 2 + 255) / 256);
   for (int f = 0; f < 120; ++f) {
@@ -607,17 +614,11 @@ int pi_backward(cvcb_lattice *L, const double *wts, double *dLdU, double *dLdmu,
 
   // adjoint solves: lambda_up = g5 Q(-mu)^-1 g5 A_up, lambda_dn = g5 Q(mu)^-1 g5 A_dn
   double *C = static_cast<double *>(cvc), *B = static_cast<double *>(bsrc);
-  for (int f = 0; f < 120; ++f) {
-    CVCB_TRY(launch_g5(L, A + f * fs, g.V));
-    CVCB_TRY(spinor_out(L, B + f * fstride, A + f * fs, g.V));
-  }
+  CVCB_TRY(spinors_out(L, B, A, 120, true));
   int rc = solve_columns(L, C, B, &S.params, -L->mu, L->mu, 60, 60, fstride);
   if (rc < 0) return rc;
   double2 *Lam = A;  // reuse
-  for (int f = 0; f < 120; ++f) {
-    CVCB_TRY(spinor_in(L, Lam + f * fs, C + f * fstride, g.V));
-    CVCB_TRY(launch_g5(L, Lam + f * fs, g.V));
-  }
+  CVCB_TRY(spinors_in(L, Lam, C, 120, true));
   // dL/dmu, dL/dkappa
   DotPairs dp;
   for (int f = 0; f < 120; ++f) {
@@ -661,18 +662,15 @@ int pi_backward(cvcb_lattice *L, const double *wts, double *dLdU, double *dLdmu,
       k_force<0><<<dim3(blocks, 4), 128, 0, L->stream>>>(G, pp, w, 0, g, ph01, ph23);
       CVCB_LAUNCHED(L);
     }
-    std::vector<double> out((size_t)72 * V);
     void *gcvc;
     CVCB_TRY(ensure_buffer(L, SLOT_ADJ_B, 72 * V * sizeof(double), &gcvc));
     k_grad_to_cvc<<<blocks, 128, 0, L->stream>>>(static_cast<double *>(gcvc), G, g);
     CVCB_LAUNCHED(L);
-    CVCB_CUDA(cudaMemcpyAsync(out.data(), gcvc, out.size() * sizeof(double),
-                              cudaMemcpyDeviceToHost, L->stream));
-    CVCB_CUDA(cudaStreamSynchronize(L->stream));
-    for (int nu = 0; nu < 4; ++nu)
-      for (int k = 0; k < 18; ++k) out[18 * (4 * (size_t)S.src + nu) + k] += gsrc[nu][k];
-    CVCB_CUDA(cudaMemcpyAsync(dLdU, out.data(), out.size() * sizeof(double), cudaMemcpyDefault,
-                              L->stream));
+    SourceGrad sg;
+    std::memcpy(sg.v, gsrc, sizeof sg.v);
+    k_add_source_grad<<<1, 96, 0, L->stream>>>(static_cast<double *>(gcvc) + 72 * (size_t)S.src, sg);
+    CVCB_LAUNCHED(L);
+    CVCB_CUDA(cudaMemcpyAsync(dLdU, gcvc, 72 * V * sizeof(double), cudaMemcpyDefault, L->stream));
     CVCB_CUDA(cudaStreamSynchronize(L->stream));
   }
   return release_columns_if_over_budget(L);

@@ -230,6 +230,9 @@ bool is_own_device_ptr(const cvcb_lattice *L, const void *p);  // memory of the 
 int spinor_in(cvcb_lattice *L, double2 *dst, const double *src, int nsites_aos);
 // Copy device-layout `src` into a CVC-layout FP64 spinor (host or device).
 int spinor_out(cvcb_lattice *L, double *dst, const double2 *src, int nsites_aos);
+// n contiguous fields in device memory (24 V doubles each) at once, times g5 if asked to.
+int spinors_in(cvcb_lattice *L, double2 *dst, const double *src, int n, bool g5);
+int spinors_out(cvcb_lattice *L, double *dst, const double2 *src, int n, bool g5);
 // Slots used by spinor_in/out staging
 enum BufSlot {
   SLOT_STAGE_A = 0,

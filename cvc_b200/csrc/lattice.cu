@@ -68,11 +68,15 @@ int ensure_buffer(cvcb_lattice *L, int slot, size_t bytes, void **out) {
 constexpr int kTile = 64;
 constexpr int kTilePad = 13;  // row pitch of the tile (12 + 1 against bank conflicts)
 
-// all V sites of dst are written: sites lex >= nsites become zero
+// all V sites of dst are written: sites lex >= nsites become zero.  Both
+// kernels take one field per blockIdx.y (V sites each), and multiply by g5 if
+// asked to.
 __global__ void __launch_bounds__(128) k_spinor_aos_to_eo(double2 *__restrict__ dst,
                                                          const double2 *__restrict__ src, Geom g,
-                                                         int nsites) {
+                                                         int nsites, bool g5) {
   __shared__ double2 t[kTile * kTilePad];
+  src += (size_t)blockIdx.y * 12 * g.V;
+  dst += (size_t)blockIdx.y * 12 * g.V;
   const int base = blockIdx.x * kTile;
   const int nloc = min(kTile, g.V - base);
   for (int q = threadIdx.x; q < nloc * 12; q += blockDim.x) {
@@ -82,21 +86,25 @@ __global__ void __launch_bounds__(128) k_spinor_aos_to_eo(double2 *__restrict__ 
   __syncthreads();
   for (int q = threadIdx.x; q < nloc * 12; q += blockDim.x) {
     const int k = q / nloc, s = q - k * nloc;
-    dst[(size_t)k * g.V + lex_to_eo(g, base + s)] = t[s * kTilePad + k];
+    const double2 v = t[s * kTilePad + k];
+    dst[(size_t)k * g.V + lex_to_eo(g, base + s)] = g5 && k >= 6 ? make_double2(-v.x, -v.y) : v;
   }
 }
 
 // sites lex < nsites of dst are written
 __global__ void __launch_bounds__(128) k_spinor_eo_to_aos(double2 *__restrict__ dst,
                                                          const double2 *__restrict__ src, Geom g,
-                                                         int nsites) {
+                                                         int nsites, bool g5) {
   __shared__ double2 t[kTile * kTilePad];
+  src += (size_t)blockIdx.y * 12 * g.V;
+  dst += (size_t)blockIdx.y * 12 * g.V;
   const int base = blockIdx.x * kTile;
   const int nloc = min(kTile, nsites - base);
   if (nloc <= 0) return;
   for (int q = threadIdx.x; q < nloc * 12; q += blockDim.x) {
     const int k = q / nloc, s = q - k * nloc;
-    t[s * kTilePad + k] = src[(size_t)k * g.V + lex_to_eo(g, base + s)];
+    const double2 v = src[(size_t)k * g.V + lex_to_eo(g, base + s)];
+    t[s * kTilePad + k] = g5 && k >= 6 ? make_double2(-v.x, -v.y) : v;
   }
   __syncthreads();
   for (int q = threadIdx.x; q < nloc * 12; q += blockDim.x) {
@@ -117,7 +125,21 @@ int spinor_in(cvcb_lattice *L, double2 *dst, const double *src, int nsites) {
                               cudaMemcpyHostToDevice, L->stream));
     dsrc = static_cast<const double2 *>(st);
   }
-  k_spinor_aos_to_eo<<<(g.V + kTile - 1) / kTile, 128, 0, L->stream>>>(dst, dsrc, g, nsites);
+  k_spinor_aos_to_eo<<<(g.V + kTile - 1) / kTile, 128, 0, L->stream>>>(dst, dsrc, g, nsites, false);
+  CVCB_LAUNCHED(L);
+  return CVCB_OK;
+}
+
+int spinors_in(cvcb_lattice *L, double2 *dst, const double *src, int n, bool g5) {
+  k_spinor_aos_to_eo<<<dim3((L->g.V + kTile - 1) / kTile, n), 128, 0, L->stream>>>(
+      dst, reinterpret_cast<const double2 *>(src), L->g, L->g.V, g5);
+  CVCB_LAUNCHED(L);
+  return CVCB_OK;
+}
+
+int spinors_out(cvcb_lattice *L, double *dst, const double2 *src, int n, bool g5) {
+  k_spinor_eo_to_aos<<<dim3((L->g.V + kTile - 1) / kTile, n), 128, 0, L->stream>>>(
+      reinterpret_cast<double2 *>(dst), src, L->g, L->g.V, g5);
   CVCB_LAUNCHED(L);
   return CVCB_OK;
 }
@@ -126,14 +148,14 @@ int spinor_out(cvcb_lattice *L, double *dst, const double2 *src, int nsites) {
   const Geom &g = L->g;
   if (is_device_ptr(dst)) {
     k_spinor_eo_to_aos<<<(g.V + kTile - 1) / kTile, 128, 0, L->stream>>>(
-        reinterpret_cast<double2 *>(dst), src, g, nsites);
+        reinterpret_cast<double2 *>(dst), src, g, nsites, false);
     CVCB_LAUNCHED(L);
     return CVCB_OK;
   }
   void *st;
   CVCB_TRY(ensure_buffer(L, SLOT_STAGE_B, (size_t)g.V * 24 * sizeof(double), &st));
   k_spinor_eo_to_aos<<<(g.V + kTile - 1) / kTile, 128, 0, L->stream>>>(static_cast<double2 *>(st), src,
-                                                                  g, nsites);
+                                                                  g, nsites, false);
   CVCB_LAUNCHED(L);
   CVCB_CUDA(cudaMemcpyAsync(dst, st, (size_t)nsites * 24 * sizeof(double),
                             cudaMemcpyDeviceToHost, L->stream));
