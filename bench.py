@@ -414,16 +414,14 @@ def main():
                               "rhs_per_thread": shape[2].value,
                               "variant": ["per-thread links", "shared-memory links",
                                           "packed FP32x2 rhs pairs", "pair-tiled fields",
-                                          "pair-tiled fields, TMEM accumulator",
-                                          "pair-tiled fields, TMEM accumulator, pipelined",
-                                          "pair-tiled fields, bulk-staged t/x neighbours"]
+                                          "pair-tiled fields, directions on warps"]
                                          [shape[3].value]},
             "inner_iterations_per_step": iters // max(args.steps, 1),
             "max_true_residual": worst_res,
         },
         "roofline": {
             "kernel": ["k_eo_hop", "k_eo_hop_staged", "k_eo_hop_x2", "k_eo_hop_pt",
-                       "k_eo_hop_ptm", "k_eo_hop_ptm", "k_eo_hop_ptb"][shape[3].value] +
+                       "k_eo_hop_sp"][shape[3].value] +
                       " (batched even/odd stencil sweep, "
                       f"{args.precision}, {params.link_recon}-real links)",
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
