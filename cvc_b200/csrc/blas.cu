@@ -73,7 +73,7 @@ int apply_full(cvcb_lattice *L, double *xi, const double *phi, double a, double 
   CVCB_TRY(launch_tm_full_cvc(L, out, in, a, b, c, g5out));
   if (!out_dev) CVCB_CUDA(cudaMemcpyAsync(xi, out, fb, cudaMemcpyDeviceToHost, L->stream));
   CVCB_CUDA(cudaStreamSynchronize(L->stream));
-  return CVCB_OK;
+  return tm_full_cvc_status(L);
 }
 
 // Stage one CVC-layout field (host or device) to a device pointer usable by

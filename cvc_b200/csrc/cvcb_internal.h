@@ -187,6 +187,8 @@ struct cvcb_lattice {
   // mapped pinned mailbox for the solver's per-rhs control values (host and
   // device addresses of the same memory), created on first use
   double *mbox_host = nullptr, *mbox_dev = nullptr;
+  // mapped pinned flag that k_tm_full_cvc sets when a wait of its runs out
+  int *late_host = nullptr, *late_dev = nullptr;
   bool have_gauge = false;
   double unitarity = -1.0;
   std::vector<double> gauge_host;  // raw CVC-layout copy (for re-phasing)
@@ -269,6 +271,7 @@ int tm_full_blocks(const Geom &g);  // partial sums of a TmDot: 3 per block
 // the same on CVC-layout device arrays (16-byte aligned, not overlapping)
 int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a, double b, double c,
                        bool g5out);
+int tm_full_cvc_status(cvcb_lattice *L);  // once the stream is synchronised
 int launch_g5(cvcb_lattice *L, double2 *f, int nsites);
 int launch_one_pm_imu_inv(cvcb_lattice *L, double2 *f, double sign, int nsites);
 

@@ -209,11 +209,7 @@ int launch_tm_full(cvcb_lattice *L, double2 *out, const double2 *in, double a, d
 // layout, which cost two field passes more than the operator itself.  Thread =
 // lexicographic site; a spinor is six 32-byte loads (one whole sector each; V4)
 // or twelve 16-byte ones (fields off a 32-byte boundary).  Same terms in the
-// same order as k_tm_full_f64: the same bits.  A call takes 29 us at
-// 22 x 14 x 10 x 18 (44 with the two copies) and 613 (818) at 32^3 x 64;
-// compulsory traffic there 2.0 GB, 0.31 ms.  Bound by L1: the strided spinor
-// loads keep its data pipe 82 % busy, and so does a copy through shared memory
-// by cp.async (644 us).
+// same order as k_tm_full_f64: the same bits.
 template <bool V4>
 __device__ __forceinline__ Spinor<double> load_spinor_cvc(const double2 *__restrict__ f, int lex) {
   const double2 *q = f + (size_t)lex * 12;
@@ -253,13 +249,106 @@ __device__ __forceinline__ void store_spinor_cvc(double2 *f, int lex, const Spin
   }
 }
 
-constexpr int kCvcThreads = 128;
+constexpr int kCvcThreads = 128, kCvcWarps = kCvcThreads / 32;
+constexpr int kCvcStage = 32 * 12;  // double2: the spinors of a warp's 32 sites in one direction
+constexpr int kCvcSmem = kCvcWarps * 2 * kCvcStage * (int)sizeof(double2);  // 48 KB
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) {
+  return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+
+// The spinors at lex index j of every lane's site into the warp's stage, in
+// lane order: one bulk copy for each run of consecutive indices (a direction's
+// neighbours of 32 consecutive sites are one run but for the periodic wraps).
+__device__ __forceinline__ void cvc_fetch(double2 *stage, unsigned long long *bar,
+                                          const double2 *__restrict__ in, int j, int lane) {
+  const int before = __shfl_up_sync(0xffffffffu, j, 1);
+  const bool first = lane == 0 || j != before + 1;
+  const unsigned starts = __ballot_sync(0xffffffffu, first);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (lane == 0)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
+                 "r"((unsigned)(kCvcStage * sizeof(double2)))
+                 : "memory");
+  __syncwarp();
+  if (first) {
+    const unsigned later = lane == 31 ? 0u : starts >> (lane + 1);
+    const int len = later ? __ffs(later) : 32 - lane;
+    asm volatile(
+        "cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+            smem_addr(stage + lane * 12)),
+        "l"(in + (size_t)j * 12), "r"(len * 192), "r"(smem_addr(bar))
+        : "memory");
+  }
+}
+__device__ __forceinline__ bool cvc_landed(unsigned long long *bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_addr(bar)), "r"(parity)
+      : "memory");
+  return ok;
+}
+// until the stage's copies have landed, for every lane; false after two seconds
+__device__ __forceinline__ bool cvc_wait(unsigned long long *bar, unsigned parity) {
+  if (__all_sync(0xffffffffu, cvc_landed(bar, parity))) return true;
+  unsigned long long t0, t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+  do {
+    if (__all_sync(0xffffffffu, cvc_landed(bar, parity))) return true;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  } while (!__any_sync(0xffffffffu, t - t0 > 2000000000ull));
+  return false;
+}
+// A lane's spinor.  Its 192 bytes start on one of two bank quarters, so lanes
+// read their components from different starting points (lane / 2 mod 4) and
+// rotate them into place afterwards: no bank conflicts.
+__device__ __forceinline__ Spinor<double> cvc_spinor(const double2 *stage, int lane) {
+  const int d = (lane >> 1) & 3;
+  const double2 *q = stage + lane * 12;
+  double2 v[12], w[12];
+#pragma unroll
+  for (int k = 0; k < 12; ++k) v[k] = q[k + d < 12 ? k + d : k + d - 12];
+#pragma unroll
+  for (int k = 0; k < 12; ++k) {
+    w[k].x = d & 1 ? v[(k + 11) % 12].x : v[k].x;
+    w[k].y = d & 1 ? v[(k + 11) % 12].y : v[k].y;
+  }
+  Spinor<double> s;
+#pragma unroll
+  for (int k = 0; k < 12; ++k)
+    s.c[k / 3][k % 3] = cx(d & 2 ? w[(k + 10) % 12].x : w[k].x, d & 2 ? w[(k + 10) % 12].y : w[k].y);
+  return s;
+}
+
+// A warp has 32 consecutive sites.  Their neighbours in a direction are brought
+// into shared memory by bulk copies, two directions ahead of the arithmetic, and
+// every lane reads its own from there.  Loads from the fields directly, 32 bytes
+// a lane and 192 apart, keep the L1 data pipe 82 % busy: 29.4 us a call at
+// 22 x 14 x 10 x 18 and 588 at 32^3 x 64, now 27.6 and 523 (with copies to and
+// from the device layout 44 and 818); compulsory traffic there 2.0 GB, 0.31 ms.
+// cp.async instead of bulk copies: 644.  More stages cost L1, which the links
+// need: three 605, four 646.  Padding against bank conflicts instead of the
+// rotation makes the copies small: 557 in fours, 581 in pairs.  A tile of the
+// block's own sites for z, y and the diagonal term: 537.
 template <bool G5OUT, bool V4>
 __global__ void __launch_bounds__(kCvcThreads, 3)
     k_tm_full_cvc(double2 *__restrict__ out, const double2 *__restrict__ in,
-                  const double2 *__restrict__ U, Geom g, double a, double b, double c) {
-  const int lex = blockIdx.x * kCvcThreads + threadIdx.x;
-  if (lex >= g.V) return;
+                  const double2 *__restrict__ U, Geom g, double a, double b, double c, int *late) {
+  extern __shared__ __align__(128) double2 cvc_sm[];
+  __shared__ unsigned long long bars[kCvcWarps][2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double2 *const st = cvc_sm + warp * 2 * kCvcStage;
+  unsigned long long *const bar = bars[warp];
+  const int want = blockIdx.x * kCvcThreads + threadIdx.x;
+  if (want - lane >= g.V) return;  // the whole warp
+  const bool valid = want < g.V;
+  const int lex = valid ? want : g.V - 1;  // idle lanes take part in the copies
+  if (lane < 2)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar + lane)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncwarp();
   SiteCoord cd;
   {
     const unsigned r0 = fdiv((unsigned)lex, g.dLZ), r1 = fdiv(r0, g.dLY), r2 = fdiv(r1, g.dLX);
@@ -278,20 +367,31 @@ __global__ void __launch_bounds__(kCvcThreads, 3)
   for (int sp = 0; sp < 4; ++sp)
 #pragma unroll
     for (int co = 0; co < 3; ++co) acc.c[sp][co] = cx(0.0, 0.0);
+  cvc_fetch(st, bar, in, nb_lex(g, cd, 0, -1), lane);
+  cvc_fetch(st + kCvcStage, bar + 1, in, nb_lex(g, cd, 0, +1), lane);
 #pragma unroll
-  for (int mu = 0; mu < 4; ++mu) {
-    {
-      const int j = nb_lex(g, cd, mu, -1);
-      const HalfSpinor<double> h = project(mu, +1, load_spinor_cvc<V4>(in, j));
-      accum_recon(mu, +1, acc, link_dag_mul(load_link64(U, V, mu, qoff + (j >> 1)), h));
+  for (int d = 0; d < 8; ++d) {  // t-, t+, x-, x+, ...
+    const int mu = d >> 1;
+    const bool fwd = d & 1;
+    const Link<double> W = load_link64(U, V, mu, fwd ? self : qoff + (nb_lex(g, cd, mu, -1) >> 1));
+    if (!cvc_wait(bar + (d & 1), (d >> 1) & 1)) {
+      *late = 1;
+      cvc_wait(bar + (1 - (d & 1)), ((d + 1) >> 1) & 1);  // the copies in flight
+      return;
     }
-    {
-      const int j = nb_lex(g, cd, mu, +1);
-      const HalfSpinor<double> h = project(mu, -1, load_spinor_cvc<V4>(in, j));
-      accum_recon(mu, -1, acc, link_mul(load_link64(U, V, mu, self), h));
-    }
+    const HalfSpinor<double> h = project(mu, fwd ? -1 : +1, cvc_spinor(st + (d & 1) * kCvcStage, lane));
+    __syncwarp();  // every lane has read the stage
+    if (d < 7)
+      cvc_fetch(st + (d & 1) * kCvcStage, bar + (d & 1), in,
+                d == 6 ? lex : nb_lex(g, cd, (d + 2) >> 1, fwd ? +1 : -1), lane);
+    accum_recon(mu, fwd ? -1 : +1, acc, fwd ? link_mul(W, h) : link_dag_mul(W, h));
   }
-  const Spinor<double> f = load_spinor_cvc<V4>(in, lex);
+  if (!cvc_wait(bar, 0)) {  // the fifth use of stage 0
+    *late = 1;
+    return;
+  }
+  const Spinor<double> f = cvc_spinor(st, lane);
+  if (!valid) return;
   Spinor<double> r;
 #pragma unroll
   for (int sp = 0; sp < 4; ++sp) {
@@ -315,7 +415,7 @@ __global__ void __launch_bounds__(kCvcThreads, 3)
 // spinor in shared memory, warps 0..2 sum the sink colours 0..2 in the order
 // of the kernels above (the same bits) and add the diagonal.
 constexpr int kCvcSplitThreads = 256;
-// Up to here: 14.2 against 16.7 us a call at 512 sites, 15.5 against 17.5 at
+// Up to here: 14.2 against 16.7 us a call at 512 sites, 16.1 against 18.4 at
 // 8192; at 12,000 18.8 against 18.2, at 55,440 32.6 against 27.
 constexpr int kCvcSplitSites = 8192;
 
@@ -425,9 +525,19 @@ int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a,
   } else {
     auto kern = g5out ? (v4 ? k_tm_full_cvc<true, true> : k_tm_full_cvc<true, false>)
                       : (v4 ? k_tm_full_cvc<false, true> : k_tm_full_cvc<false, false>);
-    kern<<<blocks, kCvcThreads, 0, L->stream>>>(o, i, L->U64, g, a, b, c);
+    CVCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvcSmem));
+    kern<<<blocks, kCvcThreads, kCvcSmem, L->stream>>>(o, i, L->U64, g, a, b, c, L->late_dev);
   }
   CVCB_LAUNCHED(L);
+  return CVCB_OK;
+}
+
+// An expired wait of the kernel above; for good, since later calls may overlap.
+int tm_full_cvc_status(cvcb_lattice *L) {
+  if (*static_cast<volatile int *>(L->late_host)) {
+    set_error("a copy of the operator's neighbours did not land in time");
+    return CVCB_ERR_CUDA;
+  }
   return CVCB_OK;
 }
 

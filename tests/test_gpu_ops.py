@@ -134,14 +134,16 @@ def test_errors(cb):
     lat.close()
 
 
-@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 4, 10), (4, 2, 14, 6), (6, 10, 14, 12)],
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 6, 4, 10), (4, 2, 14, 6), (6, 10, 14, 12),
+                                  (14, 2, 10, 34), (2, 2, 2, 1030)],
                          ids=lambda d: "x".join(map(str, d)))
 @pytest.mark.parametrize("where", ["host", "device", "device16", "to_host", "in_place"])
 def test_operator_on_cvc_fields(cb, oracle_mod, dims, where):
     """The operator on site-major arrays, below and above the volume up to which
     a site's directions go to eight warps: extents of two (both hops reach the
-    same site), a last block that is not full, fields on 32- and on 16-byte
-    boundaries, mixed memories, and input and output the same array."""
+    same site), rows that cross warps, a last block and a last warp that are not
+    full, fields on 32- and on 16-byte boundaries, mixed memories, and input and
+    output the same array."""
     torch = pytest.importorskip("torch")
     bc = (1.0, 0.0, 0.25, 0.5)
     lat = cb.Lattice(*dims, kappa=0.14, mu=0.03, bc_angle=bc)
