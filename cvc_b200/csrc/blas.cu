@@ -49,7 +49,8 @@ int need_gauge(cvcb_lattice *L) {
 
 // out = op(in) with the full-lattice kernel on CVC-layout fields, in place on
 // device arrays; host arrays go through staging, and so does an input that
-// overlaps the output.
+// overlaps the output or is managed or another GPU's memory (the kernel's bulk
+// copies read this GPU's own).
 int apply_full(cvcb_lattice *L, double *xi, const double *phi, double a, double b, double c,
                bool g5out) {
   CVCB_TRY(need_gauge(L));
@@ -61,7 +62,7 @@ int apply_full(cvcb_lattice *L, double *xi, const double *phi, double a, double 
   const double *in = phi;
   double *out = xi;
   void *f;
-  if (!is_device_ptr(phi) || (out_dev && x < p + fb && p < x + fb)) {
+  if (!is_own_device_ptr(L, phi) || (out_dev && x < p + fb && p < x + fb)) {
     CVCB_TRY(ensure_buffer(L, SLOT_F0, fb, &f));
     CVCB_CUDA(cudaMemcpyAsync(f, phi, fb, cudaMemcpyDefault, L->stream));
     in = static_cast<const double *>(f);
