@@ -1869,20 +1869,26 @@ int sloppy_normal_op(cvcb_lattice *L, int prec, int recon, int layout, int n,
                      : sloppy_normal_op_t<F16Acc, F32Acc, L32f>(L, prec, recon, n, in, out);
 }
 
-// Inner iterations on pair-tiled fields (k_eo_hop_pt and the pair CG kernels),
-// the default for FP32 and FP16 storage; CVCB_PAIRS=0 selects the per-rhs
-// fields with the packed-pair stencil k_eo_hop_x2 instead (read once per
-// process).  FP16: 12 columns at 16^3x32 take 21.5 ms against 23.7 with the
-// per-rhs fields (M^+M 220 against 247 us), whose links are FP16 too; the pair
-// kernels read the FP32 ones, shared by the pair.  A sweep takes as long as
-// in FP32 with half the requests and bytes: latency at 16 warps per SM and
-// the FMA pipe (50 % busy) bound it, not its traffic.
-bool use_pairs() {
-  static const bool on = [] {
+// Whether a batch of n right-hand sides takes pair-tiled fields (k_eo_hop_pt
+// and the pair CG kernels) for its inner iterations, or the per-rhs ones with
+// k_eo_hop and k_eo_hop_x2.  CVCB_PAIRS=0 and 1 (read once per process) pin
+// the answer for FP32 and FP16; otherwise FP32 takes pairs, and FP16 where no
+// lane of a pair idles: 12 columns at 16^3x32 take 21.5 ms against 23.7 with
+// the per-rhs fields (M^+M 220 against 247 us), whose links are FP16 too; the
+// pair kernels read the FP32 ones, shared by the pair.  A sweep takes as long
+// as in FP32 with half the requests and bytes: latency at 16 warps per SM and
+// the FMA pipe (50 % busy) bound it, not its traffic.  A lone last right-hand
+// side costs a whole pair and is stored two bytes at a time: at 16^3x32 one
+// column takes 7.8 ms in pairs and 4.4 with the per-rhs fields, 3 columns 10.3
+// and 8.1, 9 columns 19.5 and 18.4, 15 columns 28.0 and 28.1.
+constexpr int kOddPairs = 16;
+bool use_pairs(int prec, int n) {
+  static const int pinned = [] {
     const char *e = getenv("CVCB_PAIRS");
-    return !e || atoi(e) != 0;
+    return !e ? -1 : atoi(e) != 0 ? 1 : 0;
   }();
-  return on;
+  if (prec == CVCB_PREC_DOUBLE || pinned == 0) return false;
+  return pinned == 1 || prec == CVCB_PREC_SINGLE || n % 2 == 0 || n > kOddPairs;
 }
 
 int time_stencil(cvcb_lattice *L, int kind, int prec, int recon, int nrhs, int reps, double *ms) {
@@ -1918,10 +1924,11 @@ int time_stencil(cvcb_lattice *L, int kind, int prec, int recon, int nrhs, int r
   }
   if (prec == CVCB_PREC_DOUBLE)
     return time_stencil_t<F64Acc, F64Acc, L64>(L, kind, prec, 18, nrhs, reps, ms);
-  if (prec == CVCB_PREC_SINGLE && use_pairs())
+  const bool pairs = use_pairs(prec, nrhs);
+  if (prec == CVCB_PREC_SINGLE && pairs)
     return recon == 12 ? time_stencil_t<P32, P32, LT32c>(L, kind, prec, recon, nrhs, reps, ms)
                        : time_stencil_t<P32, P32, LT32f>(L, kind, prec, recon, nrhs, reps, ms);
-  if (use_pairs())
+  if (pairs)
     return recon == 12 ? time_stencil_t<P16, P32, LT32c>(L, kind, prec, recon, nrhs, reps, ms)
                        : time_stencil_t<P16, P32, LT32f>(L, kind, prec, recon, nrhs, reps, ms);
   if (prec == CVCB_PREC_SINGLE)
@@ -2071,7 +2078,7 @@ int solve_batched(cvcb_lattice *L, double *const *x, const double *const *b, int
     host_fields = !is_device_ptr(x[i]) && !is_device_ptr(b[i]);
   int nb = P->block_rhs;
   if (!nb) {
-    const bool pairs = P->precision != CVCB_PREC_DOUBLE && use_pairs();
+    const bool pairs = use_pairs(P->precision, 2);  // the candidates are even
     auto key = std::make_tuple(L->g.V,
                                P->precision + (pairs ? kPairKey : 0) + (host_fields ? 100 : 0),
                                recon, nrhs);
@@ -2101,12 +2108,13 @@ int solve_batched(cvcb_lattice *L, double *const *x, const double *const *b, int
   }
   st->batch_rhs = nb;
   auto run = [&](double *const *xs, const double *const *bs, int n, cudaEvent_t read) {
+    const bool pairs = use_pairs(P->precision, n);
     if (P->precision == CVCB_PREC_DOUBLE)
       return run_batch<F64Acc, F64Acc, L64>(L, xs, bs, n, P, st, nullptr, read);
-    if (P->precision == CVCB_PREC_SINGLE && use_pairs())
+    if (P->precision == CVCB_PREC_SINGLE && pairs)
       return recon == 12 ? run_batch<P32, P32, LT32c>(L, xs, bs, n, P, st, nullptr, read)
                          : run_batch<P32, P32, LT32f>(L, xs, bs, n, P, st, nullptr, read);
-    if (use_pairs())
+    if (pairs)
       return recon == 12 ? run_batch<P16, P32, LT32c>(L, xs, bs, n, P, st, nullptr, read)
                          : run_batch<P16, P32, LT32f>(L, xs, bs, n, P, st, nullptr, read);
     if (P->precision == CVCB_PREC_SINGLE)
@@ -2168,7 +2176,7 @@ int cvcb_tuned_shape(cvcb_lattice *L, int precision, int link_recon, int nrhs, i
                      int *rows_per_block, int *rhs_per_thread, int *variant) {
   if (!L || !sites_per_block || !rows_per_block || !rhs_per_thread || !variant)
     return CVCB_ERR_NULL;
-  const bool pairs = precision != CVCB_PREC_DOUBLE && cvcb::use_pairs();
+  const bool pairs = cvcb::use_pairs(precision, nrhs);
   auto it = cvcb::g_tuned_shape.find(std::make_tuple(
       L->g.V, precision + (pairs ? cvcb::kPairKey : 0), link_recon, nrhs));
   if (it == cvcb::g_tuned_shape.end()) {

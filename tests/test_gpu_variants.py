@@ -138,3 +138,43 @@ def test_directions_on_warps_same_bits(tmp_path, dims):
             assert abs(int(a[k][0]) - int(b[k][0])) <= 3 + 0.1 * a[k][0], k
         else:
             assert np.max(np.abs(a[k] - b[k])) <= 1e-8 * np.max(np.abs(a[k])), k
+
+
+ODD_CHILD = r"""
+import ctypes, json, os, sys
+import numpy as np
+for v in ("CVCB_SHAPE", "CVCB_PAIRS"):
+    os.environ.pop(v, None)
+sys.path.insert(0, sys.argv[1])
+import cvc_b200 as cb
+dims = (8, 4, 4, 6)
+lat = cb.Lattice(*dims, kappa=0.14, mu=0.02)
+lat.upload_gauge(cb.gauge_random(*dims, 0.3, 3))
+V = lat.VOLUME
+out = {}
+for n in (1, 2, 3, 15, 17):
+    bs = []
+    for i in range(n):
+        b = np.zeros(24 * V); b[24 * (11 * i % V) + 2 * (i % 12)] = 1.0; bs.append(b)
+    xs = [np.zeros(24 * V) for _ in range(n)]
+    p = cb.solver_defaults(); p.precision = cb.PREC_HALF; p.block_rhs = n
+    st = lat.solve(xs, bs, p)
+    v = [ctypes.c_int() for _ in range(4)]
+    rc = lat._lib.cvcb_tuned_shape(lat._h, cb.PREC_HALF, 12, n, *[ctypes.byref(q) for q in v])
+    r = np.zeros(24 * V); lat.Q_phi_tbc(r, xs[-1])
+    out[n] = [rc, v[3].value, st.converged, float(np.linalg.norm(r - bs[-1]))]
+print(json.dumps(out))
+"""
+
+
+def test_half_takes_pairs_only_where_no_lane_idles():
+    """FP16 batches of an odd number of columns up to 15 run on the per-rhs
+    fields (in pairs one column took up to twice the time), even and larger
+    ones on pair-tiled fields (variant 3 of cvcb_tuned_shape)."""
+    r = subprocess.run([sys.executable, "-c", ODD_CHILD, str(ROOT)], capture_output=True, text=True,
+                       timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    for n, (rc, variant, conv, res) in json.loads(r.stdout.strip().splitlines()[-1]).items():
+        n = int(n)
+        assert rc == 0 and conv == n and res <= 1e-10, (n, rc, conv, res)
+        assert (variant == 3) == (n % 2 == 0 or n > 15), (n, variant)
