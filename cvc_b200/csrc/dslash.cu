@@ -290,7 +290,8 @@ __device__ __forceinline__ bool cvc_landed(unsigned long long *bar, unsigned par
       : "memory");
   return ok;
 }
-// until the stage's copies have landed, for every lane; false after two seconds
+// until the stage's copies have landed, for every lane; false after two
+// seconds (looked at once more then: the warp may have been paused in between)
 __device__ __forceinline__ bool cvc_wait(unsigned long long *bar, unsigned parity) {
   if (__all_sync(0xffffffffu, cvc_landed(bar, parity))) return true;
   unsigned long long t0, t;
@@ -299,7 +300,7 @@ __device__ __forceinline__ bool cvc_wait(unsigned long long *bar, unsigned parit
     if (__all_sync(0xffffffffu, cvc_landed(bar, parity))) return true;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   } while (!__any_sync(0xffffffffu, t - t0 > 2000000000ull));
-  return false;
+  return __all_sync(0xffffffffu, cvc_landed(bar, parity));
 }
 // A lane's spinor.  Its 192 bytes start on one of two bank quarters, so lanes
 // read their components from different starting points (lane / 2 mod 4) and
@@ -532,9 +533,12 @@ int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a,
   return CVCB_OK;
 }
 
-// An expired wait of the kernel above; for good, since later calls may overlap.
+// An expired wait of the call that has just been synchronised (a lattice has
+// one call at a time); the next call starts afresh.
 int tm_full_cvc_status(cvcb_lattice *L) {
-  if (*static_cast<volatile int *>(L->late_host)) {
+  volatile int *late = L->late_host;
+  if (*late) {
+    *late = 0;
     set_error("a copy of the operator's neighbours did not land in time");
     return CVCB_ERR_CUDA;
   }
