@@ -1,5 +1,7 @@
 // Reductions behind spinor_scalar_product_co/_re (invert_Qtm.c:28-84) and
 // the C-ABI entry points of the operators.
+#include <time.h>
+
 #include <cmath>
 
 #include "cvcb_internal.h"
@@ -47,6 +49,13 @@ int need_gauge(cvcb_lattice *L) {
   return CVCB_OK;
 }
 
+// a clock of some milliseconds' resolution, read without a system call
+double coarse_seconds() {
+  timespec t;
+  clock_gettime(CLOCK_MONOTONIC_COARSE, &t);
+  return (double)t.tv_sec + 1e-9 * (double)t.tv_nsec;
+}
+
 // out = op(in) with the full-lattice kernel on CVC-layout fields, in place on
 // device arrays; host arrays go through staging, and so does an input that
 // overlaps the output or is managed or another GPU's memory (the kernel's bulk
@@ -71,10 +80,12 @@ int apply_full(cvcb_lattice *L, double *xi, const double *phi, double a, double 
     CVCB_TRY(ensure_buffer(L, SLOT_F1, fb, &f));
     out = static_cast<double *>(f);
   }
+  const double t0 = coarse_seconds();
   CVCB_TRY(launch_tm_full_cvc(L, out, in, a, b, c, g5out));
   if (!out_dev) CVCB_CUDA(cudaMemcpyAsync(xi, out, fb, cudaMemcpyDeviceToHost, L->stream));
   CVCB_CUDA(cudaStreamSynchronize(L->stream));
-  return tm_full_cvc_status(L);
+  // half the limit leaves room for two clocks that differ
+  return coarse_seconds() - t0 > 0.5 * kCvcWaitSeconds ? tm_full_cvc_status(L) : CVCB_OK;
 }
 
 // Stage one CVC-layout field (host or device) to a device pointer usable by

@@ -187,8 +187,6 @@ struct cvcb_lattice {
   // mapped pinned mailbox for the solver's per-rhs control values (host and
   // device addresses of the same memory), created on first use
   double *mbox_host = nullptr, *mbox_dev = nullptr;
-  // mapped pinned flag that k_tm_full_cvc sets when a wait of its runs out
-  int *late_host = nullptr, *late_dev = nullptr;
   bool have_gauge = false;
   double unitarity = -1.0;
   std::vector<double> gauge_host;  // raw CVC-layout copy (for re-phasing)
@@ -205,7 +203,7 @@ struct cvcb_lattice {
 
   // reduction scratch: per-block partials, a completion counter, results
   double *partials = nullptr;  // [kMaxRedBlocks * 4]
-  unsigned *red_counter = nullptr;
+  unsigned *red_counter = nullptr;  // [16]: 0 the counter, kLateFlag below
   double *red_result = nullptr;  // [8]
   cvcb::SolverScalars *scal = nullptr;
 
@@ -223,6 +221,8 @@ struct cvcb_lattice {
 namespace cvcb {
 
 constexpr int kMaxRedBlocks = 1184;  // 8 x 148 SMs
+// entry of red_counter that k_tm_full_cvc sets when a wait of its runs out
+constexpr int kLateFlag = 8;
 
 // lattice.cu
 int ensure_buffer(cvcb_lattice *L, int slot, size_t bytes, void **out);
@@ -271,7 +271,10 @@ int tm_full_blocks(const Geom &g);  // partial sums of a TmDot: 3 per block
 // the same on CVC-layout device arrays (16-byte aligned, not overlapping)
 int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a, double b, double c,
                        bool g5out);
-int tm_full_cvc_status(cvcb_lattice *L);  // once the stream is synchronised
+// once the stream is synchronised; waits give up after kCvcWaitSeconds, so that
+// a call that took less holds none that did and need not ask
+constexpr double kCvcWaitSeconds = 2.0;
+int tm_full_cvc_status(cvcb_lattice *L);
 int launch_g5(cvcb_lattice *L, double2 *f, int nsites);
 int launch_one_pm_imu_inv(cvcb_lattice *L, double2 *f, double sign, int nsites);
 

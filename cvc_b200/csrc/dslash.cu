@@ -290,8 +290,9 @@ __device__ __forceinline__ bool cvc_landed(unsigned long long *bar, unsigned par
       : "memory");
   return ok;
 }
-// until the stage's copies have landed, for every lane; false after two
-// seconds (looked at once more then: the warp may have been paused in between)
+// until the stage's copies have landed, for every lane; false after
+// kCvcWaitSeconds (looked at once more then: the warp may have been paused in
+// between)
 __device__ __forceinline__ bool cvc_wait(unsigned long long *bar, unsigned parity) {
   if (__all_sync(0xffffffffu, cvc_landed(bar, parity))) return true;
   unsigned long long t0, t;
@@ -299,7 +300,7 @@ __device__ __forceinline__ bool cvc_wait(unsigned long long *bar, unsigned parit
   do {
     if (__all_sync(0xffffffffu, cvc_landed(bar, parity))) return true;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  } while (!__any_sync(0xffffffffu, t - t0 > 2000000000ull));
+  } while (!__any_sync(0xffffffffu, t - t0 > (unsigned long long)(1e9 * kCvcWaitSeconds)));
   return __all_sync(0xffffffffu, cvc_landed(bar, parity));
 }
 // A lane's spinor.  Its 192 bytes start on one of two bank quarters, so lanes
@@ -336,7 +337,7 @@ __device__ __forceinline__ Spinor<double> cvc_spinor(const double2 *stage, int l
 template <bool G5OUT, bool V4>
 __global__ void __launch_bounds__(kCvcThreads, 3)
     k_tm_full_cvc(double2 *__restrict__ out, const double2 *__restrict__ in,
-                  const double2 *__restrict__ U, Geom g, double a, double b, double c, int *late) {
+                  const double2 *__restrict__ U, Geom g, double a, double b, double c, unsigned *late) {
   extern __shared__ __align__(128) double2 cvc_sm[];
   __shared__ unsigned long long bars[kCvcWarps][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -527,7 +528,7 @@ int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a,
     auto kern = g5out ? (v4 ? k_tm_full_cvc<true, true> : k_tm_full_cvc<true, false>)
                       : (v4 ? k_tm_full_cvc<false, true> : k_tm_full_cvc<false, false>);
     CVCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvcSmem));
-    kern<<<blocks, kCvcThreads, kCvcSmem, L->stream>>>(o, i, L->U64, g, a, b, c, L->late_dev);
+    kern<<<blocks, kCvcThreads, kCvcSmem, L->stream>>>(o, i, L->U64, g, a, b, c, L->red_counter + kLateFlag);
   }
   CVCB_LAUNCHED(L);
   return CVCB_OK;
@@ -536,9 +537,12 @@ int launch_tm_full_cvc(cvcb_lattice *L, double *out, const double *in, double a,
 // An expired wait of the call that has just been synchronised (a lattice has
 // one call at a time); the next call starts afresh.
 int tm_full_cvc_status(cvcb_lattice *L) {
-  volatile int *late = L->late_host;
-  if (*late) {
-    *late = 0;
+  unsigned late = 0;
+  unsigned *const flag = L->red_counter + kLateFlag;
+  CVCB_CUDA(cudaMemcpyAsync(&late, flag, sizeof late, cudaMemcpyDeviceToHost, L->stream));
+  CVCB_CUDA(cudaStreamSynchronize(L->stream));
+  if (late) {
+    CVCB_CUDA(cudaMemsetAsync(flag, 0, sizeof late, L->stream));
     set_error("a copy of the operator's neighbours did not land in time");
     return CVCB_ERR_CUDA;
   }

@@ -321,12 +321,6 @@ int cvcb_lattice_create(cvcb_lattice **out, int T, int LX, int LY, int LZ, int d
   if (e == cudaSuccess) e = cudaMemset(L->red_counter, 0, 16 * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc(&L->red_result, 8 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&L->scal, sizeof(SolverScalars));
-  if (e == cudaSuccess)
-    e = cudaHostAlloc(reinterpret_cast<void **>(&L->late_host), sizeof(int), cudaHostAllocMapped);
-  if (e == cudaSuccess) {
-    *L->late_host = 0;
-    e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&L->late_dev), L->late_host, 0);
-  }
   if (e != cudaSuccess) {
     set_error("context set-up failed: %s", cudaGetErrorString(e));
     cvcb_lattice_destroy(L);
@@ -360,7 +354,6 @@ int cvcb_lattice_destroy(cvcb_lattice *L) {
   for (cudaEvent_t e : L->pipe_ev)
     if (e) cudaEventDestroy(e);
   if (L->mbox_host) cudaFreeHost(L->mbox_host);
-  if (L->late_host) cudaFreeHost(L->late_host);
   if (L->stream) cudaStreamDestroy(L->stream);
   delete L;
   return CVCB_OK;

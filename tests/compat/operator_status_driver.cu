@@ -16,7 +16,8 @@ int main() {
   for (size_t k = 0; k < phi.size(); ++k) phi[k] = 1.0 / (1.0 + k % 97);
   if (cvcb_Q_phi_tbc(L, xi.data(), phi.data()) != CVCB_OK) return 2;
   const std::vector<double> want = xi;
-  *L->late_host = 1;
+  const unsigned one = 1;
+  cudaMemcpy(L->red_counter + cvcb::kLateFlag, &one, sizeof one, cudaMemcpyHostToDevice);
   const int late = cvcb::tm_full_cvc_status(L);
   const int next = cvcb_Q_phi_tbc(L, xi.data(), phi.data());
   std::printf("%d %d %d\n", late == CVCB_ERR_CUDA, next == CVCB_OK, xi == want);

@@ -169,3 +169,35 @@ def test_operator_on_cvc_fields(cb, oracle_mod, dims, where):
         got = y if isinstance(y, np.ndarray) else y.cpu().numpy()
         assert rel_err(got, getattr(orc, name)(phi, *extra)) < 1e-14
     lat.close()
+
+
+def test_lattice_set_up_pins_no_memory(cb):
+    """Making a lattice and freeing it takes less than one pinned allocation
+    and its release alone, which it therefore cannot contain."""
+    import ctypes
+    import time
+    torch = pytest.importorskip("torch")
+    torch.zeros(1, device="cuda")
+    lib = ctypes.CDLL([line.split()[-1] for line in open("/proc/self/maps") if "libcudart" in line][0])
+    p = ctypes.c_void_p()
+
+    def pinned():
+        assert lib.cudaHostAlloc(ctypes.byref(p), ctypes.c_size_t(4), 2) == 0
+        assert lib.cudaFreeHost(p) == 0
+
+    def median(fn):
+        t = []
+        for _ in range(25):
+            t0 = time.perf_counter()
+            fn()
+            t.append(time.perf_counter() - t0)
+        return sorted(t)[12]
+
+    def lattice():
+        cb.Lattice(8, 4, 4, 4).close()
+
+    lattice()
+    pinned()
+    made, pin = median(lattice), median(pinned)
+    print(f"lattice {1e6 * made:.0f} us, pinned allocation {1e6 * pin:.0f} us")
+    assert made < pin
