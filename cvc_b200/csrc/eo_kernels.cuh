@@ -381,15 +381,16 @@ __device__ __forceinline__ unsigned warp_mask() {
   const int t = threadIdx.y * blockDim.x + threadIdx.x, left = blockDim.x * blockDim.y - (t & ~31);
   return left >= 32 ? 0xffffffffu : (1u << left) - 1;
 }
-// partials of a row of bx threads (one rhs; whole warps, or 16 lanes each)
-__host__ __device__ inline int res_parts(int bx) { return bx < 32 ? 1 : bx / 32; }
+// one partial per 16 sites, whatever the block's shape (rows of 16 or of whole
+// warps), so that the sums do not depend on the shape that the tuner took
+__host__ __device__ inline int res_parts(int Vh) { return (Vh + 15) / 16; }
 template <class SF, class LF>
 __device__ __forceinline__ void store_res_part(const HopArgs<SF, LF> &A, int r, bool act, double n2,
-                                               int sb) {
-  const int w = blockDim.x < 32 ? blockDim.x : 32;
-  for (int o = w >> 1; o > 0; o >>= 1) n2 += __shfl_down_sync(warp_mask(), n2, o, w);
-  if (act && (threadIdx.x & (w - 1)) == 0)
-    A.dot_part[(size_t)r * A.dot_np + A.dot_off + sb * res_parts(blockDim.x) + threadIdx.x / w] = n2;
+                                               int i) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) n2 += __shfl_down_sync(warp_mask(), n2, o, 16);
+  if (act && (threadIdx.x & 15) == 0 && i < A.eg.g.Vh)
+    A.dot_part[(size_t)r * A.dot_np + A.dot_off + i / 16] = n2;
 }
 
 template <class SF, class LF, int NR, bool G5IN, bool G5HOP, bool AUX, int RES = 0>
@@ -411,10 +412,7 @@ __device__ __forceinline__ void eo_hop_body(const HopArgs<SF, LF> &A) {
   for (int sb = blockIdx.y; sb * (int)blockDim.x < g.Vh; sb += gridDim.y) {
     const int i = sb * blockDim.x + threadIdx.x;
     if (RES) {  // the whole warp takes part in the sum of the norm
-      if (__all_sync(warp_mask(), i >= g.Vh)) {
-        store_res_part(A, r0, true, 0.0, sb);
-        continue;
-      }
+      if (__all_sync(warp_mask(), i >= g.Vh)) continue;
     } else if (i >= g.Vh) {
       return;
     }
@@ -465,7 +463,7 @@ __device__ __forceinline__ void eo_hop_body(const HopArgs<SF, LF> &A) {
 #pragma unroll
         for (int q = 0; q < 3; ++q) o.c[s][q] = c * acc[k].c[s][q];
       if constexpr (RES != 0) {
-        store_res_part(A, r0, true, i < g.Vh ? hop_epilogue<RES>(A, r0, i, o) : 0.0, sb);
+        store_res_part(A, r0, true, i < g.Vh ? hop_epilogue<RES>(A, r0, i, o) : 0.0, i);
         continue;
       }
       o = diag_op((R)A.d1a, (R)A.d1b, o);
@@ -831,7 +829,7 @@ __device__ __forceinline__ void eo_hop_staged_body(const HopArgs<SF, LF> &A) {
         A.out.store(r, i, o);
       }
     }
-    if (RES) store_res_part(A, r, act, n2, sb);
+    if (RES) store_res_part(A, r, act, n2, i);
     __syncthreads();  // the next site block overwrites the staged links
   }
 }

@@ -347,19 +347,25 @@ __device__ __forceinline__ void diag_pair(SpinorPair &o, const SpinorPair &v, co
     }
 }
 
-// |v|^2 of one site for both right-hand sides, accumulated in FP64
+// |v|^2 of one site for both right-hand sides, in FP64: the components of a
+// colour in the order of their spins, then the colours 0, 1, 2.  Both sweeps
+// below sum in this order, and take one partial per 32-site tile, so that alpha
+// and beta do not depend on which of them the tuner took.
+__device__ __forceinline__ void add_norm2(double2 &n, const CP &z) {
+  n.x = fma((double)z.re.x, (double)z.re.x, n.x);
+  n.x = fma((double)z.im.x, (double)z.im.x, n.x);
+  n.y = fma((double)z.re.y, (double)z.re.y, n.y);
+  n.y = fma((double)z.im.y, (double)z.im.y, n.y);
+}
 __device__ __forceinline__ double2 norm2_pair(const SpinorPair &v) {
   double2 n = make_double2(0.0, 0.0);
 #pragma unroll
-  for (int s = 0; s < 4; ++s)
+  for (int c = 0; c < 3; ++c) {
+    double2 t = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const CP &z = v.c[s][c];
-      n.x = fma((double)z.re.x, (double)z.re.x, n.x);
-      n.x = fma((double)z.im.x, (double)z.im.x, n.x);
-      n.y = fma((double)z.re.y, (double)z.re.y, n.y);
-      n.y = fma((double)z.im.y, (double)z.im.y, n.y);
-    }
+    for (int s = 0; s < 4; ++s) add_norm2(t, v.c[s][c]);
+    n = make_double2(n.x + t.x, n.y + t.y);
+  }
   return n;
 }
 
@@ -567,7 +573,7 @@ static_assert(kSplitThreads == kRedThreads, "the last block reduces with block_s
 template <class LF, bool G5IN, bool G5HOP, bool AUX, bool RUPD = false>
 __global__ void __launch_bounds__(kSplitThreads) k_eo_hop_sp(const __grid_constant__ HopArgs<P32, LF> A) {
   __shared__ float4 sh[8][6][kTile];
-  __shared__ double2 sn[3];
+  __shared__ double2 sn[3][kTile];  // |out|^2 per colour and site
   const int pr = blockIdx.x, ra = 2 * pr;
   const bool act_a = !(A.done && A.done[ra]);
   const bool has_b = ra + 1 < A.nrhs;
@@ -645,8 +651,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_eo_hop_sp(const __grid_consta
             rv.im = __ffma2_rn(na, o.im, rv.im);
             o = rv;
           }
-          n2.x = fma((double)o.re.x, (double)o.re.x, fma((double)o.im.x, (double)o.im.x, n2.x));
-          n2.y = fma((double)o.re.y, (double)o.re.y, fma((double)o.im.y, (double)o.im.y, n2.y));
+          add_norm2(n2, o);
           float4 *q = dst + P32::comp(3 * s + warp);
           if (act_a && act_b) {
             *q = f4_of(o);
@@ -657,19 +662,21 @@ __global__ void __launch_bounds__(kSplitThreads) k_eo_hop_sp(const __grid_consta
           }
         }
       }
-      if (A.dot_part) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          n2.x += __shfl_down_sync(0xffffffffu, n2.x, o);
-          n2.y += __shfl_down_sync(0xffffffffu, n2.y, o);
-        }
-        if (lane == 0) sn[warp] = n2;
-      }
+      if (A.dot_part) sn[warp][lane] = n2;
     }
     __syncthreads();  // also: the next tile overwrites sh
-    if (A.dot_part && threadIdx.x == 0) {
-      A.dot_part[(size_t)ra * A.dot_np + tile] = sn[0].x + sn[1].x + sn[2].x;
-      if (has_b) A.dot_part[(size_t)(ra + 1) * A.dot_np + tile] = sn[0].y + sn[1].y + sn[2].y;
+    if (A.dot_part && warp == 0) {
+      double da = sn[0][lane].x + sn[1][lane].x + sn[2][lane].x;
+      double db = sn[0][lane].y + sn[1][lane].y + sn[2][lane].y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        da += __shfl_down_sync(0xffffffffu, da, o);
+        db += __shfl_down_sync(0xffffffffu, db, o);
+      }
+      if (lane == 0) {
+        A.dot_part[(size_t)ra * A.dot_np + tile] = da;
+        if (has_b) A.dot_part[(size_t)(ra + 1) * A.dot_np + tile] = db;
+      }
     }
   }
   if (!A.dot_part || !A.fin.kind) return;

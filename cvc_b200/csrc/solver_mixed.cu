@@ -1066,10 +1066,7 @@ struct Batch {
     sh.by = std::min(sh.by, n);
     return sh;
   }
-  int res_np() const {
-    const LaunchShape sh = shape_f64();
-    return (g.Vh + sh.bx - 1) / sh.bx * res_parts(sh.bx);
-  }
+  int res_np() const { return res_parts(g.Vh); }
   template <int RES>
   int hop64_res(HopArgs<F64Acc, L64> a, int np, int off) {
     const LaunchShape sh = shape_f64();

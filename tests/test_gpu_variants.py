@@ -178,3 +178,52 @@ def test_half_takes_pairs_only_where_no_lane_idles():
         n = int(n)
         assert rc == 0 and conv == n and res <= 1e-10, (n, rc, conv, res)
         assert (variant == 3) == (n % 2 == 0 or n > 15), (n, variant)
+
+
+BITS_CHILD = r"""
+import sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+sys.path.insert(0, sys.argv[1] + "/tests")
+import cvc_b200 as cb
+from conftest import seeded
+dims, prec = tuple(int(v) for v in sys.argv[3].split("x")), int(sys.argv[4])
+lat = cb.Lattice(*dims, kappa=0.14, mu=0.02, bc_angle=(1.0, 0.0, 0.5, 0.0))
+lat.upload_gauge(cb.gauge_random(*dims, 0.3, 3))
+V = lat.VOLUME
+bs = [seeded(20 + i, 24 * V) for i in range(15)]
+xs = [np.zeros(24 * V) for _ in bs]
+p = cb.solver_defaults()
+p.precision = prec
+st = []
+for k, n in [(i, 1) for i in range(12)] + [(12, 3)]:
+    p.block_rhs = n
+    s = lat.solve(xs[k:k + n], bs[k:k + n], p)
+    assert s.converged == n
+    st += [s.iterations, s.max_true_res]
+np.savez(sys.argv[2], x=np.array(xs), st=np.array(st))
+"""
+
+
+@pytest.mark.parametrize("dims", ["2x2x6x10", "8x6x8x10"])
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+def test_solve_bits_do_not_depend_on_the_shape(tmp_path, prec, dims):
+    """Two processes whose tuners take different shapes return the same bits,
+    of the solutions and of the residuals: the norms behind alpha, beta and the
+    residuals sum in one order for every shape (rows of 16 sites and of whole
+    warps, one thread or eight warps a site), on half volumes of 120 and 1920
+    sites, for lone columns and three together."""
+    import numpy as np
+    shapes = (["64,1,1", "16,1,1", "16,3,1", "32,3,1", "128,1,1"] if prec == 0 else
+              ["64,1,2,1", "32,1,2,2", "32,2,2,1", "256,1,2,1"])
+    got = []
+    for shape in shapes:
+        f = tmp_path / (shape.replace(",", "_") + ".npz")
+        out = subprocess.run([sys.executable, "-c", BITS_CHILD, str(ROOT), str(f), dims, str(prec)],
+                             env=dict(os.environ, CVCB_SHAPE=shape, CVCB_PAIRS="1"),
+                             capture_output=True, text=True, timeout=600)
+        assert out.returncode == 0, out.stderr[-2000:]
+        got.append(np.load(f))
+    for shape, g in zip(shapes[1:], got[1:]):
+        assert np.array_equal(g["st"], got[0]["st"]), (shape, g["st"] - got[0]["st"])
+        assert np.array_equal(g["x"], got[0]["x"]), shape
