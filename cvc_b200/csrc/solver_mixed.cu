@@ -1376,6 +1376,10 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
         f.nr = 2;
         f.pk = nf >= 4 && f.pk == 2 && std::is_same<SF, P32>::value ? 2 : 1;
         if (f.pk == 2) f.bx = kTile, f.by = 1;
+        if (std::is_same<SF, P16>::value && f.bx % 32) {  // whole warps; the per-rhs FP16 fields
+          f.bx += 32 - f.bx % 32;                         // take any width, so none is refused here
+          f.by = std::max(1, std::min(f.by, kHopMaxThreads / f.bx));
+        }
       }
       B.shape = f;
       g_tuned_shape[key] = f;

@@ -227,3 +227,12 @@ def test_solve_bits_do_not_depend_on_the_shape(tmp_path, prec, dims):
     for shape, g in zip(shapes[1:], got[1:]):
         assert np.array_equal(g["st"], got[0]["st"]), (shape, g["st"] - got[0]["st"])
         assert np.array_equal(g["x"], got[0]["x"]), shape
+
+
+def test_half_takes_rows_that_are_no_whole_warps():
+    """CVCB_SHAPE with 16 or 48 sites in a row: FP16 solves run whether their
+    fields are tiled by pairs or not."""
+    for shape in ("16,4,1", "48,1,1", "48,5,2,1"):
+        for pairs in (0, 1):
+            r = run(2, shape, pairs)
+            assert r["conv"] == 11 and r["res"] <= 1e-10 and r["chk"] <= 1e-10, (shape, pairs, r)
