@@ -412,16 +412,16 @@ def main():
             "link_recon": params.link_recon, "rhs_per_batch": nb,
             "stencil_shape": {"sites_per_block": shape[0].value, "rows_per_block": shape[1].value,
                               "rhs_per_thread": shape[2].value,
-                              "variant": ["per-thread links", "shared-memory links",
-                                          "packed FP32x2 rhs pairs", "pair-tiled fields",
-                                          "pair-tiled fields, directions on warps"]
+                              "variant": {0: "per-thread links", 1: "shared-memory links",
+                                          2: "packed FP32x2 rhs pairs", 3: "pair-tiled fields",
+                                          7: "pair-tiled fields, directions on warps"}
                                          [shape[3].value]},
             "inner_iterations_per_step": iters // max(args.steps, 1),
             "max_true_residual": worst_res,
         },
         "roofline": {
-            "kernel": ["k_eo_hop", "k_eo_hop_staged", "k_eo_hop_x2", "k_eo_hop_pt",
-                       "k_eo_hop_sp"][shape[3].value] +
+            "kernel": {0: "k_eo_hop", 1: "k_eo_hop_staged", 2: "k_eo_hop_x2", 3: "k_eo_hop_pt",
+                       7: "k_eo_hop_sp"}[shape[3].value] +
                       " (batched even/odd stencil sweep, "
                       f"{args.precision}, {params.link_recon}-real links)",
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",

@@ -2188,7 +2188,7 @@ int cvcb_tuned_shape(cvcb_lattice *L, int precision, int link_recon, int nrhs, i
   *sites_per_block = s.bx;
   *rows_per_block = s.by;
   *rhs_per_thread = s.nr;
-  *variant = pairs ? (s.pk == 2 ? 4 : 3) : s.pk ? 2 : (s.by > 1 && s.nr == 1) ? 1 : 0;
+  *variant = pairs ? (s.pk == 2 ? 7 : 3) : s.pk ? 2 : (s.by > 1 && s.nr == 1) ? 1 : 0;
   return CVCB_OK;
 }
 

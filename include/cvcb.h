@@ -286,9 +286,9 @@ int cvcb_time_link_product(cvcb_lattice *lat, int variant, int reps, double *ms,
  * thread rows per block (each row a group of right-hand sides), right-hand
  * sides per thread, and the kernel variant (0: links per thread, 1: links
  * staged in shared memory for all rows, 2: two rhs per thread in packed
- * FP32x2 arithmetic, 3: pair-tiled fields, 4: pair-tiled fields with a site's
- * eight directions on eight warps); CVCB_ERR_STATE
- * before the first tuning. */
+ * FP32x2 arithmetic, 3: pair-tiled fields, 7: pair-tiled fields with a site's
+ * eight directions on eight warps; 4 to 6 stood for kernels that are gone and
+ * are not used again); CVCB_ERR_STATE before the first tuning. */
 int cvcb_tuned_shape(cvcb_lattice *lat, int precision, int link_recon, int nrhs,
                      int *sites_per_block, int *rows_per_block, int *rhs_per_thread,
                      int *variant);

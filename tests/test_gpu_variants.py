@@ -236,3 +236,28 @@ def test_half_takes_rows_that_are_no_whole_warps():
         for pairs in (0, 1):
             r = run(2, shape, pairs)
             assert r["conv"] == 11 and r["res"] <= 1e-10 and r["chk"] <= 1e-10, (shape, pairs, r)
+
+
+CODE_CHILD = r"""
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import cvc_b200 as cb
+lat = cb.Lattice(8, 4, 4, 4, kappa=0.14, mu=0.02)
+lat.upload_gauge(cb.gauge_random(8, 4, 4, 4, 0.3, 3))
+b = np.zeros(24 * 512); b[0] = 1.0
+lat.solve([np.zeros(24 * 512)], [b])
+v = [ctypes.c_int() for _ in range(4)]
+lat._lib.cvcb_tuned_shape(lat._h, cb.PREC_SINGLE, 12, 1, *[ctypes.byref(q) for q in v])
+print(*[q.value for q in v])
+"""
+
+
+@pytest.mark.parametrize("shape,want", [("64,1,2,1", [64, 1, 2, 3]), ("32,1,2,2", [32, 1, 2, 7])])
+def test_variant_codes(shape, want):
+    """cvcb_tuned_shape names the kernel that a pinned shape runs; the codes 4
+    to 6 of kernels that are gone do not come back with another meaning."""
+    r = subprocess.run([sys.executable, "-c", CODE_CHILD, str(ROOT)], capture_output=True, text=True,
+                       env=dict(os.environ, CVCB_SHAPE=shape, CVCB_PAIRS="1"), timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert [int(t) for t in r.stdout.split()] == want
