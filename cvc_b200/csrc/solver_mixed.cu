@@ -1904,9 +1904,9 @@ int time_stencil(cvcb_lattice *L, int kind, int prec, int recon, int nrhs, int r
     CVCB_TRY(ensure_buffer(L, SLOT_F0, fb, &f0));
     CVCB_TRY(ensure_buffer(L, SLOT_F1, fb, &f1));
     CVCB_CUDA(cudaMemsetAsync(f0, 0, fb, L->stream));
-    auto one = [&] {
-      return launch_tm_full(L, (double2 *)f1, (const double2 *)f0, 0.5 / L->kappa, L->mu, -0.5,
-                            false, nullptr);
+    auto one = [&] {  // as cvcb_Q_phi_tbc applies it
+      return launch_tm_full_cvc(L, (double *)f1, (const double *)f0, 0.5 / L->kappa, L->mu, -0.5,
+                                false);
     };
     CVCB_TRY(one());
     cudaEvent_t a, b;
@@ -1921,7 +1921,7 @@ int time_stencil(cvcb_lattice *L, int kind, int prec, int recon, int nrhs, int r
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     *ms = t / reps;
-    return CVCB_OK;
+    return tm_full_cvc_status(L);
   }
   if (prec == CVCB_PREC_DOUBLE)
     return time_stencil_t<F64Acc, F64Acc, L64>(L, kind, prec, 18, nrhs, reps, ms);
