@@ -1836,7 +1836,11 @@ int sloppy_normal_op_t(cvcb_lattice *L, int prec, int recon, int n, const double
   CVCB_CUDA(cudaMemcpyAsync(B.S.scale, ones.data(), sizeof(double) * n, cudaMemcpyHostToDevice,
                             L->stream));
   dim3 eg((g.Vh + 127) / 128, n);
-  k_to_sloppy<<<eg, 128, 0, L->stream>>>(B.p, B.f64(B.b64, 1), B.S.scale, nullptr, g.Vh, n);
+  if constexpr (kPairTiled<SF>)
+    k_to_sloppy_pt<<<dim3(eg.x, (n + 1) / 2), 128, 0, L->stream>>>(B.p, B.f64(B.b64, 1), B.S.scale,
+                                                                    nullptr, g.Vh, n);
+  else
+    k_to_sloppy<<<eg, 128, 0, L->stream>>>(B.p, B.f64(B.b64, 1), B.S.scale, nullptr, g.Vh, n);
   CVCB_LAUNCHED(L);
   CVCB_TRY(B.normal_op_sloppy(B.Ap, B.p, nullptr));
   CVCB_CUDA(cudaMemsetAsync(B.y64, 0, fs * n * sizeof(double2), L->stream));
@@ -1855,11 +1859,14 @@ int sloppy_normal_op(cvcb_lattice *L, int prec, int recon, int layout, int n,
     return CVCB_ERR_STATE;
   }
   if (n <= 0 || n > kMaxBatch || prec < 0 || prec > 2 || (recon != 12 && recon != 18) ||
-      layout < 0 || layout > 1 || (layout == 1 && prec != CVCB_PREC_SINGLE)) {
+      layout < 0 || layout > 1 || (layout == 1 && prec == CVCB_PREC_DOUBLE)) {
     set_error("invalid arguments");
     return CVCB_ERR_ARG;
   }
   if (prec == CVCB_PREC_DOUBLE) return sloppy_normal_op_t<F64Acc, F64Acc, L64>(L, prec, 18, n, in, out);
+  if (layout == 1 && prec == CVCB_PREC_HALF)
+    return recon == 12 ? sloppy_normal_op_t<P16, P32, LT32c>(L, prec, recon, n, in, out)
+                       : sloppy_normal_op_t<P16, P32, LT32f>(L, prec, recon, n, in, out);
   if (layout == 1)
     return recon == 12 ? sloppy_normal_op_t<P32, P32, LT32c>(L, prec, recon, n, in, out)
                        : sloppy_normal_op_t<P32, P32, LT32f>(L, prec, recon, n, in, out);

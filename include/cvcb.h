@@ -263,8 +263,9 @@ int cvcb_time_stencil(cvcb_lattice *lat, int kind, int precision, int link_recon
  * odd-site Schur complement A_oo - 1/4 H_oe A_ee^-1 H_eo of Q_phi_tbc's
  * operator, M(mu)^+ = g5 M(-mu) g5), even sites of out are set to zero.  The
  * fields go through the storage of `precision` (CVCB_PREC_*) with
- * link_recon reals per link; layout 1 selects the pair-tiled FP32 storage
- * (precision CVCB_PREC_SINGLE only), layout 0 the per-rhs one.  For checking
+ * link_recon reals per link; layout 1 selects the pair-tiled storage
+ * (CVCB_PREC_SINGLE and CVCB_PREC_HALF, the latter with the FP32 links), layout
+ * 0 the per-rhs one.  For checking
  * the reduced-precision operators against the FP64 one.  No counterpart in
  * the reference. */
 int cvcb_sloppy_normal_op(cvcb_lattice *lat, int precision, int link_recon, int layout, int nrhs,

@@ -147,3 +147,40 @@ def test_batched_solve_partial_tile(cb):
         lat.Q_phi_tbc(r, x)
         assert np.linalg.norm(r - b) / np.linalg.norm(b) <= 1e-10
     lat.close()
+
+
+# FP16 fields tiled by pairs, what FP16 solves run on: the tolerance of FP16
+# storage above (a site's components are rounded to 2^-12 of its largest one,
+# five times on the way; the links are FP32).
+@pytest.mark.parametrize("recon", [12, 18])
+def test_half_pairs_operator_against_oracle(env, recon):
+    lat, ins, want = env
+    outs = [np.zeros_like(x) for x in ins]
+    lat.sloppy_normal_op(ins, outs, 2, recon, 1)  # five: the last lane of a pair idles
+    for o, w in zip(outs, want):
+        assert rel_err(o, w) < 3e-3
+
+
+@pytest.mark.parametrize("recon", [12, 18])
+def test_half_pairs_operator_partial_tile(cb, oracle_mod, recon):
+    """Fields of very different size in one pair, whose scales are their own."""
+    g = cb.gauge_random(*DIMS_PARTIAL, 0.25, 5)
+    lat = cb.Lattice(*DIMS_PARTIAL, kappa=KAPPA, mu=MU)
+    lat.upload_gauge(g)
+    orc = oracle_mod.Oracle(*DIMS_PARTIAL, KAPPA, MU)
+    orc.set_gauge(g)
+    odd = odd_mask(DIMS_PARTIAL)
+    ins = [10.0 ** (-6 * i) * seeded(700 + i, 24 * lat.VOLUME) for i in range(3)]
+    outs = [np.zeros_like(x) for x in ins]
+    lat.sloppy_normal_op(ins, outs, 2, recon, 1)
+    for x, o in zip(ins, outs):
+        w = g5(schur(orc, g5(schur(orc, x, MU, odd)), -MU, odd))
+        assert rel_err(o, w) < 3e-3
+    orc.set_params(KAPPA, MU)
+    lat.close()
+
+
+def test_pair_layout_is_refused_in_double(env):
+    lat, ins, _ = env
+    with pytest.raises(Exception):
+        lat.sloppy_normal_op(ins, [np.zeros_like(x) for x in ins], 0, 18, 1)
