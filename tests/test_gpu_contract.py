@@ -159,3 +159,30 @@ def test_pi_kernel_variants_agree(tmp_path):
         out[v] = np.load(f)
     for v in range(1, 6):
         assert np.array_equal(out[v], out[0]), (v, float(np.max(np.abs(out[v] - out[0]))))
+
+
+@pytest.mark.parametrize("dims", [(6, 6, 6, 6), (8, 6, 10, 8)], ids=lambda d: "x".join(map(str, d)))
+def test_contract_blocks_walk(cb, oracle_mod, dims):
+    """More groups of 8 sites than the GPU has SMs (162 and 480): blocks go on
+    to a second and a fourth group, with the links and columns fetched ahead
+    for them, and some end before others.  Twice, for the same bits."""
+    torch = pytest.importorskip("torch")
+    bc = (1.0, 0.3, 0.0, 0.5)
+    lat = cb.Lattice(*dims, kappa=KAPPA, mu=MU, bc_angle=bc)
+    V = lat.VOLUME
+    assert V // 8 > torch.cuda.get_device_properties(0).multi_processor_count
+    g = cb.gauge_random(*dims, 0.3, 5)
+    lat.upload_gauge(g)
+    orc = oracle_mod.Oracle(*dims, KAPPA, MU, bc)
+    orc.set_gauge(g)
+    fields = [seeded(50 + i, 24 * V) for i in range(120)]
+    src = V // 2 + 1
+    oconn, ocontact = orc.cvc_contract(fields, src)
+    given = [torch.from_numpy(f).cuda() for f in fields]
+    torch.cuda.synchronize()
+    conn, contact = lat.cvc_contract(given, src)
+    again, _ = lat.cvc_contract(given, src)
+    assert rel_err(conn, oconn) < 1e-12
+    assert np.max(np.abs(contact - ocontact)) < 1e-12 * np.max(np.abs(ocontact))
+    assert np.array_equal(conn, again)
+    lat.close()
