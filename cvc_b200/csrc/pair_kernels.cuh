@@ -118,18 +118,6 @@ struct P32 {
     }
     return s;
   }
-  __device__ __forceinline__ Spinor<float> load_raw(int r, int j, float &nm) const {
-    nm = 1.f;
-    return load(r, j);
-  }
-  __device__ __forceinline__ void store(int r, int j, const Spinor<float> &s) const {
-    float *q = reinterpret_cast<float *>(at(r >> 1, j)) + (r & 1);
-#pragma unroll
-    for (int k = 0; k < 12; ++k) {
-      q[4 * comp(k)] = s.c[k / 3][k % 3].re;
-      q[4 * comp(k) + 2] = s.c[k / 3][k % 3].im;
-    }
-  }
 };
 
 inline size_t p32_pair_float4(int Vh) { return (size_t)((Vh + kTile - 1) / kTile) * 12 * kTile; }

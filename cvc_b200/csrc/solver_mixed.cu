@@ -819,7 +819,6 @@ struct Batch {
   F64Acc f64(double2 *base, int parity) const {
     return F64Acc{base + (size_t)parity * g.Vh, (size_t)g.V, (size_t)12 * g.V};
   }
-  F64Acc f64full(double2 *base) const { return F64Acc{base, (size_t)g.V, (size_t)12 * g.V}; }
 
   // With dot_part (packed kernel only, warp-aligned blocks), the sweep also
   // writes per-warp partials of |out|^2 (dot_np per rhs).
@@ -921,7 +920,7 @@ struct Batch {
       a.rup = rs;
       a.alpha = S.alpha;
       if (finishes_dots()) a.fin = dot_finish(2);
-        Rec rec{};
+      Rec rec{};
       if (prof_rec) {
         CVCB_CUDA(cudaEventCreate(&rec.a));
         CVCB_CUDA(cudaEventCreate(&rec.b));
