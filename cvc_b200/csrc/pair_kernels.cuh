@@ -561,7 +561,11 @@ static_assert(kSplitThreads == kRedThreads, "the last block reduces with block_s
 template <class LF, bool G5IN, bool G5HOP, bool AUX, bool RUPD = false>
 __global__ void __launch_bounds__(kSplitThreads) k_eo_hop_sp(const __grid_constant__ HopArgs<P32, LF> A) {
   __shared__ float4 sh[8][6][kTile];
-  __shared__ double2 sn[3][kTile];  // |out|^2 per colour and site
+  // |out|^2 per colour and site, for warp 0 to add up in k_eo_hop_pt's order.  On
+  // lattices that fill the GPU the sweep takes 4 to 7 % longer than with a sum per
+  // colour and warp, at 8^3 x 16 and below no longer; sums per colour in
+  // k_eo_hop_pt too cost that one 0.2 % of M^+ M at 24^3 x 48.
+  __shared__ double2 sn[3][kTile];
   const int pr = blockIdx.x, ra = 2 * pr;
   const bool act_a = !(A.done && A.done[ra]);
   const bool has_b = ra + 1 < A.nrhs;

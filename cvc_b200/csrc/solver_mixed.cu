@@ -1389,6 +1389,8 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
   // for a single right-hand side (the second lane of its pair idles)
   LaunchShape best = pairs ? LaunchShape{64, 1, 2, 1} : LaunchShape{};
   float best_ms = 1e30f;
+  // pair-tiled sweeps with the norm of M p, which costs the shapes differently
+  auto op = [&] { return B.normal_op_sloppy(B.Ap, B.p, nullptr, pairs ? B.dot_part : nullptr); };
   const int bxs[] = {32, 64, 128, 256};
   const int bys[] = {1, 2, 3, 4, 6};
   // (rhs per thread, packed): 2 rhs per thread either as two unpacked
@@ -1408,7 +1410,7 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
       B.shape.nr = nr;
       B.shape.pk = np[1];
       float ms;
-      if (time_ms(L, [&] { return B.normal_op_sloppy(B.Ap, B.p, nullptr); }, 3, &ms) != CVCB_OK) {
+      if (time_ms(L, op, 3, &ms) != CVCB_OK) {
         cudaGetLastError();
         continue;
       }
@@ -1420,7 +1422,7 @@ int tune_shape(cvcb_lattice *L, Batch<SF, XF, LF> &B, int prec, int recon, int b
   if (std::is_same<SF, P32>::value) {  // a site's directions on eight warps
     B.shape = LaunchShape{kTile, 1, 2, 2};
     float ms;
-    if (time_ms(L, [&] { return B.normal_op_sloppy(B.Ap, B.p, nullptr); }, 3, &ms) != CVCB_OK)
+    if (time_ms(L, op, 3, &ms) != CVCB_OK)
       cudaGetLastError();
     else if (ms < best_ms)
       best = B.shape;
