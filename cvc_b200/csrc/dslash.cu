@@ -1,5 +1,6 @@
 // Full-lattice FP64 twisted-mass Wilson operator with per-link boundary
-// phases: the kernel behind Q_phi_tbc, Q_phi, Qf5 and Hopping.
+// phases: k_tm_full_cvc and k_tm_full_cvc_split behind Q_phi_tbc, Q_phi, Qf5
+// and Hopping, k_tm_full_f64 behind the FP64 solvers and the hopping expansion.
 //
 //   out(x) = a in(x) + i b g5 in(x)
 //          + c sum_mu [ (1 - g_mu) U_mu(x) in(x+mu) + (1 + g_mu) U_mu(x-mu)^+ in(x-mu) ]

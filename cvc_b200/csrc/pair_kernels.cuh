@@ -1,5 +1,5 @@
-// Pair-tiled storage and its kernels for the FP32 inner iterations of the
-// batched solver.
+// Pair-tiled storage and its kernels for the inner iterations of the batched
+// solver, in FP32 and, for FP16 storage, P16 below.
 //
 // Right-hand sides 2q and 2q+1 ("pair q") are stored interleaved per complex
 // spin-colour component, so that 16 bytes hold both right-hand sides of a

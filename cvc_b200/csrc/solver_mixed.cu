@@ -15,8 +15,8 @@
 //   recursion restarts from r_N = M^+ r_hat (formed in sloppy precision).
 //   |r_hat| is the residual of the full system (the even rows vanish by
 //   construction), so convergence is decided on |b - Q x| / |b| in FP64.
-//   Finally x_e = A_ee^-1 (b_e + 1/2 H_eo x_o), Q x is recomputed in FP64 on
-//   both parities and |b - Q x| / |b| is checked.
+//   Finally x_e = A_ee^-1 (b_e + 1/2 H_eo x_o), and |b - Q x| / |b| is checked
+//   in FP64: the even rows in the sweep that forms x_e, the odd rows in another.
 #include <algorithm>
 #include <atomic>
 #include <chrono>

@@ -8,8 +8,8 @@ A = 1/(2 kappa) + i mu g5.  The oracle builds it from its own Q_phi_tbc:
 y = Q x (x odd only) has y_e = -1/2 H_eo x; z = A^-1 y_e; w = Q z (z even
 only) has w_o = -1/2 H_oe z, so M x = A x - w_o; and M^+ = g5 M(-mu) g5.
 Tolerances, relative to the largest component: FP64 storage 1e-13, FP32
-(per-rhs and pair-tiled layouts, 12- and 18-real links) 1e-5, FP16+norm
-3e-3; the two FP32 layouts agree with each other to 2e-6.  An odd number of
+(per-rhs and pair-tiled layouts, 12- and 18-real links) 1e-5, FP16+norm (both
+layouts) 3e-3; the two FP32 layouts agree with each other to 2e-6.  An odd number of
 right-hand sides leaves the last pair of the pair-tiled layout half used."""
 import numpy as np
 import pytest

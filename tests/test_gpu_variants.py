@@ -3,9 +3,8 @@ child process (the autotuner caches one shape per configuration and
 process): one rhs per thread with per-thread links, shared-memory links
 for several rows, 2 and 4 rhs per thread, packed FP32x2 rhs pairs, and
 (FP32 only, CVCB_PAIRS=1) the pair-tiled fields with 12- and 18-real
-links, with plain neighbour loads, with the t and x neighbours staged in
-shared memory by bulk copies (4th shape field 2) and with the accumulator in
-tensor memory at both register budgets (4th shape field 3, 4).
+links, with a thread per site and with a site's directions on eight warps (4th
+shape field 2); other 4th fields, 3 and 4 among them, run the former.
 A wrong sloppy operator would still be corrected by the FP64 reliable
 updates, so each variant must also converge in the same number of inner
 iterations as the plain one (the arithmetic differs only in rounding)."""
